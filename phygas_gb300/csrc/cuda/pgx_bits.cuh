@@ -139,4 +139,33 @@ PGX_HD double rcp_refine(double d, double y) {
     return fma(y, fma(e, e, e), y);
 }
 
+// Reciprocal and reciprocal square root on the GPU's fast units: within 2 ulp (4 eps relative) by their documented
+// worst case (PTX rcp.approx.f32: 1 ulp; rsqrt.approx.f32: relative error 2^-22.9; both over the full range).  The
+// .ftz forms flush subnormal arguments and results, which never occur here: every argument is checked or clamped to
+// be at least 1e-30, and a reciprocal's argument at most 1e30, so arguments and results are normal -- and they issue
+// as one special-function instruction, without the subnormal scaling around it.  Host builds use the exact operations,
+// which the same margins cover, scaled by (1 + host_fast_err): a host test sets it to put the results at either end
+// of the device units' error band (it is 0 otherwise, and does not exist in device code).
+#ifndef __CUDA_ARCH__
+inline float host_fast_err = 0.f;
+#endif
+PGX_HD float fast_rcp(float x) {
+#ifdef __CUDA_ARCH__
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+#else
+    return 1.f / x * (1.f + host_fast_err);
+#endif
+}
+PGX_HD float fast_rsqrt(float x) {
+#ifdef __CUDA_ARCH__
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+#else
+    return 1.f / sqrtf(x) * (1.f + host_fast_err);
+#endif
+}
+
 }  // namespace pgx

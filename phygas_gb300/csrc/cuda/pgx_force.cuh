@@ -3,6 +3,7 @@
 #pragma once
 #include "pgx_bits.cuh"
 #include "pgx_internal.cuh"
+#include "pgx_orbit32.cuh"
 
 namespace pgx {
 
@@ -37,6 +38,32 @@ __global__ void k_halo_tables() {
     }
 }
 constexpr int kHaloTableThreads = kPowSub > kPow2N ? kPowSub : kPow2N;
+
+// the same model for the FP32 orbit (pgx_orbit32.cuh): the constants above in floats
+struct MwModel32 {
+    static constexpr double bulge_GM = kBulgeGM, disk_GM = kDiskGM, halo_GM = kHaloGM, halo_inv_a = kHaloInvA;
+    static constexpr double a = kHaloG1 - 1.0, s = -0.5 * a;
+    static constexpr float cut2 = (float)(kHaloCut * kHaloCut);
+    static constexpr float a1 = split2(s).h, a1l = split2(s).l, c2 = (float)(s * (s - 1) / 2),
+                           c3 = (float)(s * (s - 1) * (s - 2) / 6), c4 = (float)(s * (s - 1) * (s - 2) * (s - 3) / 24);
+    PGX_HD static constexpr F2 bulge_b2() { return split2(kBulgeB2); }
+    PGX_HD static constexpr F2 disk_b2() { return split2(kDiskB2); }
+    PGX_HD static constexpr F2 disk_a() { return split2(kDiskA); }
+    PGX_HD static constexpr F3 far() { return split3(kHaloFar); }       // cut p / (1 + p), p = (cut / 12)^(1 + a)
+};
+static __device__ float4 g_halo32[kHalo32N];
+struct HaloTable32 {
+    __device__ __forceinline__ Halo32 operator()(int n) const {
+        const float4 v = __ldg(&g_halo32[n]);
+        return Halo32{v.x, v.y, v.z, v.w};
+    }
+};
+__global__ void k_halo32_table() {
+    const int n = blockIdx.x * blockDim.x + threadIdx.x;
+    if (n >= kHalo32N) return;
+    const Halo32 h = halo32_entry(n, MwModel32::a, kHaloInvA);
+    g_halo32[n] = make_float4(h.i, h.u0, h.u1, h.u2);
+}
 
 // x^a for x > 0 normal (here x in [8e-14, 8.4])
 __device__ __forceinline__ double halo_pow_a(double x) {
@@ -118,6 +145,80 @@ struct Orbit {
         x = fma(vx, dt, x); y = fma(vy, dt, y); z = fma(vz, dt, z);
         mw_accel(x, y, z, ax, ay, az);
         vx = fma(ax, h, vx); vy = fma(ay, h, vy); vz = fma(az, h, vz);
+    }
+};
+
+// mw_accel and the step on four lanes per orbit: the same operations on the same operands, so the same bits, in 32 FP64
+// warp instructions a step instead of 68.  An FP64 warp instruction costs the same with one lane active or 32, so where
+// there are fewer orbits than the schedulers can use lanes, an orbit's independent operations go side by side: lane 0
+// holds x and the bulge, lane 1 y and the disk, lane 2 z and the halo, lane 3 the halo's side products.  A product is
+// issued as fma(a, b, -0.0), which rounds the same.  q: the lane's coordinate (lane 3: anything finite).
+__device__ __forceinline__ double quad_accel(double q, int role) {
+    const unsigned all = 0xffffffffu;
+    const double x = __shfl_sync(all, q, 0, 4), y = __shfl_sync(all, q, 1, 4), z = __shfl_sync(all, q, 2, 4);
+    const bool bulge = role == 0, disk = role == 1, halo = role == 2;
+    const double R2 = fma(x, x, y * y);
+    const double w = fma(z, z, disk ? kDiskB2 : R2);                      // r2, or z^2 + b^2 of the disk
+    const double arg = w + (bulge ? kBulgeB2 : 0.0);
+    const uint32_t hi = f64_hi(arg);
+    bool ok = seed_ok(hi) && (disk || __double_as_longlong(w) > kTinyR2Bits);
+    const double inv = rsqrt_refine(arg, widen_seed(rsqrtf(seed_arg(hi))));        // ib, iz, ir, ir
+    // -GM ib | a + sqrt(z^2 + b^2) | r | r, then ib^2 | D^2 | r / 12 | r / 12
+    const double A = fma(bulge ? -kBulgeGM : w, inv, disk ? kDiskA : -0.0);
+    const double Ac = disk || __double_as_longlong(A) < kHaloCutBits ? A : kHaloCut;
+    const double B = fma(bulge ? inv : Ac, bulge ? inv : (disk ? A : kHaloInvA), disk ? R2 : -0.0);
+    // the halo's table entries (lanes 2 and 3), the disk's second seed
+    const long long bits = __double_as_longlong(B);
+    int e = (int)((bits >> 52) & 0x7ff) - 1023;
+    e = e < -kPow2Bias ? -kPow2Bias : (e > kPow2N - 1 - kPow2Bias ? kPow2N - 1 - kPow2Bias : e);
+    const int j = (int)((bits >> (52 - kPowSubLog)) & (kPowSub - 1));
+    const double m = __longlong_as_double((bits & 0x000fffffffffffffLL) | 0x3ff0000000000000LL);
+    const uint32_t hB = f64_hi(B);
+    ok = ok && (!disk || seed_ok(hB));
+    const double yD = widen_seed(rsqrtf(seed_arg(hB)));
+    static_assert(kPowTerms == 4, "the series below has four terms");
+    //                          disk: 1 / D           halo: (1 + t)^a       helper: ir^3, -GM r / 12, c_j^a 2^(a e)
+    const double C1 = fma(disk ? yD : (halo ? m : inv), disk ? yD : (halo ? __ldg(&g_halo_invc[j]) : inv),
+                          halo ? -1.0 : -0.0);
+    const double t = C1;
+    const double C2 = fma(disk ? -B : (halo ? __ldg(&g_halo_coef[4]) : C1), disk || halo ? C1 : inv,
+                          disk ? 1.0 : (halo ? __ldg(&g_halo_coef[3]) : -0.0));
+    const double C3 = fma(disk || halo ? C2 : -kHaloGM, disk ? 0.375 : (halo ? t : B),
+                          disk ? 0.5 : (halo ? __ldg(&g_halo_coef[2]) : -0.0));
+    const double C4 = fma(disk ? C2 : (halo ? C3 : __ldg(&g_halo_pow2[e + kPow2Bias])),
+                          disk ? C3 : (halo ? t : __ldg(&g_halo_powc[j])), halo ? __ldg(&g_halo_coef[1]) : -0.0);
+    const double C5 = fma(disk ? yD : C4, disk ? C4 : t, disk ? yD : __ldg(&g_halo_coef[0]));
+    const double ir3 = __shfl_sync(all, C2, 3, 4), gx = __shfl_sync(all, C3, 3, 4), pw = __shfl_sync(all, C4, 3, 4);
+    const double C6 = (disk ? C5 : pw) * C5;                              // iD^2 | x^a
+    const double C7 = (disk ? C5 : B) * C6;                               // iD^3 | p
+    const double C8 = fma(disk ? -kDiskGM : 1.0, C7, disk ? -0.0 : 1.0);  // fd   | 1 + p
+    const uint32_t h8 = f64_hi(C8);
+    ok = ok && (!halo || seed_ok(h8));
+    const double y8 = widen_seed(__frcp_rn(seed_arg(h8)));
+    const double C9 = fma(disk ? C8 : -C8, disk ? kDiskA : y8, disk ? -0.0 : 1.0);       // fd a | e
+    const double q8 = C7 * fma(y8, fma(C9, C9, C9), y8);                  // p / (1 + p)
+    const double fh = __shfl_sync(all, (gx * q8) * ir3, 2, 4);
+    const double fr = fma(__shfl_sync(all, A, 0, 4), __shfl_sync(all, B, 0, 4), fh);
+    const double g = fr + __shfl_sync(all, C8, 1, 4);
+    const double gz = fma(__shfl_sync(all, C9, 1, 4), __shfl_sync(all, inv, 1, 4), g);
+    double a = (halo ? gz : g) * q;
+    if (__any_sync(all, !ok && role != 3)) {                              // an argument outside the seeds' range
+        double ax, ay, az;
+        mw_accel(x, y, z, ax, ay, az);
+        a = bulge ? ax : (disk ? ay : az);
+    }
+    return a;
+}
+
+// One coordinate of an orbit on four lanes (Orbit's step)
+struct QuadOrbit {
+    double q, v, a;
+    __device__ __forceinline__ void init(int role) { a = quad_accel(q, role); }
+    __device__ __forceinline__ void kdk(double dt, double h, int role) {
+        v = fma(a, h, v);
+        q = fma(v, dt, q);
+        a = quad_accel(q, role);
+        v = fma(a, h, v);
     }
 };
 

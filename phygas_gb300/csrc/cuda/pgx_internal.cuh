@@ -19,6 +19,7 @@ constexpr double kHaloCut = 100.0;
 constexpr long long kHaloCutBits = 0x4059000000000000LL;       // the bit pattern of kHaloCut (checked in orbit_setup)
 constexpr double kTinyR2 = 1e-24;                               // below it the force's r is taken as 1e-12
 constexpr long long kTinyR2Bits = 0x3af357c299a88ea7LL;        // the bit pattern of kTinyR2 (checked in orbit_setup)
+constexpr double kHaloFar = 89.6846708671283;                   // cut p / (1 + p), p = (cut / 12)^(gamma - 1)
 constexpr double kHaloG1 = 2.02 - 1.0;                          // gamma - 1, as the reference forms it
 constexpr double kStepMyr = 0.5;                                // PH_PRE_STEP_MYR
 constexpr int kSub = 10;                                        // PH_LIN_SUB

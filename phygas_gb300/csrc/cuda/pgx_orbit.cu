@@ -9,7 +9,7 @@
 //                  lower bound on the smallest eigenvalue of S for the filter's error bounds)
 //   k_pair_mc      persistent: warps take items of <= 32 clones of one pair from a device queue (longest first),
 //                  trace them back with KDK leapfrog and the segment closest approach (reference ph_pair_clone,
-//                  src/phygas.c:200-216); the warp that finishes a pair's last item reduces it in registers
+//                  src/phygas.c:200-216), on the FP32 and integer units where they are as accurate; the warp that finishes a pair's last item reduces it in registers
 //                  with warp shuffles (reference ph_pair_reduce, src/phygas.c:218-238)
 //   k_pair_reduce_big  the same reduction for pairs of more than 1024 clones, one CTA per pair in shared memory
 //   k_mc_prep, k_pair_mc_t, k_pair_reduce_dev  the same work as one captured CUDA graph for batches of pairs of at
@@ -187,30 +187,23 @@ __device__ __forceinline__ float norm32_hi(float x, float y, float z) {
 // approach so far (an upper bound of it in FP32, with an absolute margin for the FP64 path's own rounding), the
 // segment cannot improve it and the FP64 segment test is skipped.  Otherwise the reference's test runs as before,
 // so the results are the same bits -- and the FP64 pipe does that work only near the closest approach.
-struct Clone {
-    Orbit a, b;
+struct Nearest {
     double r0x, r0y, r0z, best, tbest, vbest;
     float f0x, f0y, f0z, n0, best_up;          // r0 truncated to FP32, |r0| from below, best from above
     __device__ __forceinline__ void set_best_up() { best_up = fmaf(f32_trunc(best), 1.f + 2.4e-7f, 1e-37f); }
-    __device__ __forceinline__ void start(const double *__restrict__ ps) {
-        a.x = ps[0]; a.y = ps[1]; a.z = ps[2]; a.vx = ps[3]; a.vy = ps[4]; a.vz = ps[5];
-        b.x = ps[6]; b.y = ps[7]; b.z = ps[8]; b.vx = ps[9]; b.vy = ps[10]; b.vz = ps[11];
-        a.init();
-        b.init();
-        r0x = a.x - b.x; r0y = a.y - b.y; r0z = a.z - b.z;
+    // r0 = the separation, (ux, uy, uz) the relative velocity at the start
+    __device__ __forceinline__ void start(double rx, double ry, double rz, double ux, double uy, double uz) {
+        r0x = rx; r0y = ry; r0z = rz;
         best = sqrt(fma(r0x, r0x, fma(r0y, r0y, r0z * r0z)));
         tbest = 0.0;
-        const double ux = a.vx - b.vx, uy = a.vy - b.vy, uz = a.vz - b.vz;
         vbest = sqrt(fma(ux, ux, fma(uy, uy, uz * uz)));
         f0x = f32_trunc(r0x); f0y = f32_trunc(r0y); f0z = f32_trunc(r0z);
         n0 = norm32_lo(f0x, f0y, f0z);
         set_best_up();
     }
-    // step i (1-based) of length dt (negative), h = dt / 2
-    __device__ __forceinline__ void step(int i, double dt, double h) {
-        a.kdk(dt, h);
-        b.kdk(dt, h);
-        const double r1x = a.x - b.x, r1y = a.y - b.y, r1z = a.z - b.z;
+    // step i (1-based) of length dt (negative) has ended at separation r1; vel() = the relative speed there
+    template <class Vel>
+    __device__ __forceinline__ void segment(int i, double dt, double r1x, double r1y, double r1z, const Vel &vel) {
         const float f1x = f32_trunc(r1x), f1y = f32_trunc(r1y), f1z = f32_trunc(r1z);
         const float n1 = norm32_lo(f1x, f1y, f1z);
         const float dn = fmaf(2.2e-7f, n0 + n1, norm32_hi(f1x - f0x, f1y - f0y, f1z - f0z));
@@ -238,8 +231,7 @@ struct Clone {
                 if (dm < best) {
                     best = dm;
                     tbest = ((double)(i - 1) + s) * -dt;
-                    const double wx = a.vx - b.vx, wy = a.vy - b.vy, wz = a.vz - b.vz;
-                    vbest = sqrt(fma(wx, wx, fma(wy, wy, wz * wz)));
+                    vbest = vel();
                     set_best_up();
                 }
             }
@@ -250,16 +242,278 @@ struct Clone {
     }
 };
 
-__device__ __forceinline__ void trace_clone(const double *__restrict__ ps, int steps, double dt, double &best_o,
-                                            double &tbest_o, double &vbest_o) {
-    Clone c;
-    c.start(ps);
+// A clone's closest approach: distance (kpc), time (Myr), speed (kpc/Myr)
+struct Approach {
+    double best, tbest, vbest;
+};
+
+// One clone per lane in FP64, one orbit after the other.
+__device__ __noinline__ Approach trace_clone64(const double *__restrict__ ps, int steps, double dt) {
+    Orbit a, b;
+    a.x = ps[0]; a.y = ps[1]; a.z = ps[2]; a.vx = ps[3]; a.vy = ps[4]; a.vz = ps[5];
+    b.x = ps[6]; b.y = ps[7]; b.z = ps[8]; b.vx = ps[9]; b.vy = ps[10]; b.vz = ps[11];
+    a.init();
+    b.init();
+    Nearest n;
+    n.start(a.x - b.x, a.y - b.y, a.z - b.z, a.vx - b.vx, a.vy - b.vy, a.vz - b.vz);
     const double h = 0.5 * dt;
 #pragma unroll 1
-    for (int i = 1; i <= steps; i++) c.step(i, dt, h);
-    best_o = c.best;
-    tbest_o = c.tbest;
-    vbest_o = c.vbest;
+    for (int i = 1; i <= steps; i++) {
+        a.kdk(dt, h);
+        b.kdk(dt, h);
+        n.segment(i, dt, a.x - b.x, a.y - b.y, a.z - b.z, [&]() {
+            const double wx = a.vx - b.vx, wy = a.vy - b.vy, wz = a.vz - b.vz;
+            return sqrt(fma(wx, wx, fma(wy, wy, wz * wz)));
+        });
+    }
+    return Approach{n.best, n.tbest, n.vbest};
+}
+
+// One clone by a whole warp in FP64 (the same bits): lanes 0-3 trace its target, 4-7 its cluster (quad_accel), the
+// others repeat them.  A step takes 32 FP64 instructions where trace_clone64 takes 136, so a warp with one or two
+// such clones ends four times sooner.
+__device__ __noinline__ Approach trace_clone64_warp(const double *__restrict__ ps, int steps, double dt) {
+    const unsigned all = 0xffffffffu;
+    const int role = threadIdx.x & 3, c = role < 3 ? role : 2;
+    const double *p = ps + (threadIdx.x & 4 ? 6 : 0);
+    QuadOrbit o;
+    o.q = role < 3 ? p[c] : 0.0;
+    o.v = role < 3 ? p[3 + c] : 0.0;
+    o.init(role);
+    Nearest n;
+    // component k of the target's orbit less the cluster's, on every lane
+    auto diff = [&](double v, int k) { return __shfl_sync(all, v, k) - __shfl_sync(all, v, 4 + k); };
+    n.start(diff(o.q, 0), diff(o.q, 1), diff(o.q, 2), diff(o.v, 0), diff(o.v, 1), diff(o.v, 2));
+    const double h = 0.5 * dt;
+#pragma unroll 1
+    for (int i = 1; i <= steps; i++) {
+        o.kdk(dt, h, role);
+        n.segment(i, dt, diff(o.q, 0), diff(o.q, 1), diff(o.q, 2), [&]() {
+            const double wx = diff(o.v, 0), wy = diff(o.v, 1), wz = diff(o.v, 2);
+            return sqrt(fma(wx, wx, fma(wy, wy, wz * wz)));
+        });
+    }
+    return Approach{n.best, n.tbest, n.vbest};
+}
+
+// ---- the clone on the FP32 and integer units (pgx_orbit32.cuh) -----------------------------------------------------
+// Two orbits of about 340 instructions a step and 50 for the closest approach: bound by the issue rate, where the FP64
+// clone above is bound by the FP64 pipe at 141.6 instructions x 19 cycles per SM a clone-step.  1,024 pulsar pairs x
+// 1,000 clones: 3.55e10 clone-steps/s against 3.5e9; 64 pairs x 200 clones x 400 steps, where a warp's latency counts,
+// 1.1 against 8.4 ms.  FP64 stays for orbits outside its range and for ties (segment64).
+//
+// The closest approach over the steps' segments r0 -> r1 = r0 + d (exact integer differences of the positions) is the
+// reference's, with most segments decided from float estimates of r1.d and r1.r1:
+//   receding   r0.d > 0 for certain: the segment's nearest point is r0, which the segment before has counted;
+//   approaching r1.d < 0 for certain: the nearest point is r1.  When it improves on the best for certain it becomes the
+//              record without being evaluated ("pending"): while the pair keeps approaching, each next r1 is nearer
+//              still.  It is evaluated when the approach ends there;
+//   otherwise  (a minimum inside the step, a few per clone, or an undecided sign) the reference's test in FP64.
+// The float errors, in units of a position's high word (2^-23 kpc): each component of r1 and d is within 2^-23 relative
+// or 2^-24 absolute, so with |r1|, |d| > 8 r1.d is within 2^-21.3 |r1||d| and r0.d = r1.d - d.d within 2^-21.3 (|r1||d| +
+// d.d); both signs are certain where the square exceeds 2^-40 d.d (r1.r1 + d.d).  Squared distances are compared with a
+// relative margin of 2^-19.  Shorter vectors (10^-6 kpc) take the FP64 test.
+constexpr float kSure2 = 0x1p-40f, kSureUp = 1.f + 0x1p-19f, kSureDown = 1.f - 0x1p-19f, kSureMin = 64.f;
+
+struct I3 {
+    long long x, y, z;
+};
+__device__ __forceinline__ I3 operator-(const I3 &a, const I3 &b) { return I3{a.x - b.x, a.y - b.y, a.z - b.z}; }
+// in units of the high word, within 2^-23 relative
+__device__ __forceinline__ float fixed_to_f32(long long v) {
+    return fmaf((float)(unsigned)v, 0x1p-32f, (float)(int)(v >> 32));
+}
+__device__ __forceinline__ double norm64(const I3 &v) {
+    const double x = (double)v.x, y = (double)v.y, z = (double)v.z;
+    return sqrt(fma(x, x, fma(y, y, z * z)));
+}
+
+// The segment test of step i (1-based) in FP64: r1, d = r1 - r0 in position units of u kpc, v2 = twice the relative
+// displacement at the step's end in units of u / 64 kpc.  at_r0: the best is at r0 and unevaluated.  r0's distance is
+// counted already: only a point beyond it can improve (s > 0).
+//
+// A minimum within a hair of an end of its step: the reference compares the two steps' distances, which differ by less
+// than FP64 resolves, and which of them is the record (the time is the same, the speed is that at the end of the
+// record's step) is decided by the rounding of its FP64 orbits.  *tie = the step after which the FP64 trace decides it
+// (kTie: seven roundings of 2^-53, as a relative difference of the distances, doubled for squares).
+constexpr double kTie = 0x1p-50;
+enum { kSegNone, kSegBest, kSegAtR0 };
+
+__device__ __noinline__ int segment64(const I3 r1, const I3 d, const I3 v2, int i, double dt, double u, bool at_r0,
+                                      Approach &b, int *tie) {
+    const double dx = (double)d.x, dy = (double)d.y, dz = (double)d.z;
+    const I3 r0 = r1 - d;
+    const double rx = (double)r0.x, ry = (double)r0.y, rz = (double)r0.z;
+    const double dd = fma(dx, dx, fma(dy, dy, dz * dz)), an = fma(rx, dx, fma(ry, dy, rz * dz));
+    const int none = at_r0 ? kSegAtR0 : kSegNone;
+    if (!(dd > 0) || !(an < 0)) return none;
+    const double s = fmin(-an / dd, 1.0);
+    const double mx = fma(dx, s, rx), my = fma(dy, s, ry), mz = fma(dz, s, rz);
+    const double m2 = fma(mx, mx, fma(my, my, mz * mz)), dm = sqrt(m2) * u;
+    const bool hair = at_r0 ? s < 1.0 && an * an < kTie * dd * m2 : fabs(dm - b.best) < kTie * dm;
+    if (!at_r0 && !hair && !(dm < b.best)) return none;
+    *tie = s < 1.0 && (an + dd) * (an + dd) < kTie * dd * m2 ? i + 1 : (hair ? i : 0);
+    b.best = dm;
+    b.tbest = ((double)(i - 1) + s) * -dt;
+    b.vbest = norm64(v2) * (u * (1.0 / 128.0)) / fabs(dt);
+    return kSegBest;
+}
+
+// The record at the end of step i: both orbits there, their displacements those of the next drift
+__device__ __noinline__ Approach vertex64(const Orbit32 a, const Orbit32 b, const Force32 K, const OrbitScale s, int i,
+                                          double dt) {
+    float r2;
+    const HaloTable32 T;
+    const Acc64i A = accel32<MwModel32>(K, T, s.c, a.x, a.y, a.z, r2), B = accel32<MwModel32>(K, T, s.c, b.x, b.y, b.z, r2);
+    const double u = ldexp(1.0, s.e - 55);
+    const I3 v2 = {2 * (a.wx - b.wx) - (A.x - B.x), 2 * (a.wy - b.wy) - (A.y - B.y),
+                   2 * (a.wz - b.wz) - (A.z - B.z)};                 // 2 v dt = 2 w - a dt^2
+    return Approach{norm64(I3{a.x - b.x, a.y - b.y, a.z - b.z}) * u, (double)i * -dt,
+                    norm64(v2) * (u * (1.0 / 128.0)) / fabs(dt)};
+}
+
+struct Clone32 {
+    Orbit32 a, b;
+    Force32 K;
+    OrbitScale s;
+    Approach r;
+    float q, rmax;           // r.best^2 in squared high-word units; r2 limit
+    int tie;                 // > 0: the record is a tie that the FP64 trace of this many steps decides
+    bool pend, ok;
+    __device__ __forceinline__ double unit() const { return __hiloint2double((1023 - 55 + s.e) << 20, 0); }
+    __device__ __forceinline__ void set_q() {
+        const float f = (float)(r.best * __hiloint2double((1023 + 23 - s.e) << 20, 0));
+        q = f * f;
+    }
+    // false: not an orbit for these units (traced in FP64)
+    __device__ __forceinline__ bool start(const double *__restrict__ ps, int steps, double dt) {
+        double p[12];
+#pragma unroll
+        for (int j = 0; j < 12; j++) p[j] = ps[j];
+        double reach = 0.0;
+#pragma unroll
+        for (int o = 0; o < 12; o += 6) {
+            const double x = fmax(fabs(p[o]), fmax(fabs(p[o + 1]), fabs(p[o + 2])));
+            const double v = fmax(fabs(p[o + 3]), fmax(fabs(p[o + 4]), fabs(p[o + 5]))) * fabs(dt);
+            reach = fmax(reach, fmax(2.0 * x + 2.0 * v * steps + 20.0, 256.0 * v));
+        }
+        double sum = 0.0;                                     // NaN and infinities, which fmax passes over
+#pragma unroll
+        for (int j = 0; j < 12; j++) sum += p[j];
+        if (!(fabs(sum) < 1e300)) reach = sum * 0.0 + 1e300;
+        pend = false;
+        tie = 0;
+        ok = orbit32_scale(reach, dt, s);
+        if (!ok) return false;
+        K = force32_constants<MwModel32>(dt, s);
+        rmax = orbit32_max_r2(s);
+        float ra, rb;
+        orbit32_start<MwModel32>(a, K, HaloTable32(), s, p, p + 3, dt, ra);
+        orbit32_start<MwModel32>(b, K, HaloTable32(), s, p + 6, p + 9, dt, rb);
+        in_range(ra, rb);
+        const double rx = p[0] - p[6], ry = p[1] - p[7], rz = p[2] - p[8];
+        r.best = sqrt(fma(rx, rx, fma(ry, ry, rz * rz)));
+        r.tbest = 0.0;
+        const double ux = p[3] - p[9], uy = p[4] - p[10], uz = p[5] - p[11];
+        r.vbest = sqrt(fma(ux, ux, fma(uy, uy, uz * uz)));
+        set_q();
+        return true;
+    }
+    __device__ __forceinline__ void in_range(float ra, float rb) {
+        ok = ok && fmaxf(ra, rb) < rmax && fminf(ra, rb) > kOrbit32MinR2;
+    }
+    __device__ __forceinline__ void step(int i, double dt) {
+        const I3 sa = {a.wx >> 6, a.wy >> 6, a.wz >> 6}, sb = {b.wx >> 6, b.wy >> 6, b.wz >> 6};
+        a.x += sa.x; a.y += sa.y; a.z += sa.z;
+        b.x += sb.x; b.y += sb.y; b.z += sb.z;
+        float ra, rb;
+        const HaloTable32 T;
+        const Acc64i A = accel32<MwModel32>(K, T, s.c, a.x, a.y, a.z, ra);
+        const Acc64i B = accel32<MwModel32>(K, T, s.c, b.x, b.y, b.z, rb);
+        in_range(ra, rb);
+        const I3 d = sa - sb, r1 = {a.x - b.x, a.y - b.y, a.z - b.z};
+        const float dx = fixed_to_f32(d.x), dy = fixed_to_f32(d.y), dz = fixed_to_f32(d.z);
+        const float rx = fixed_to_f32(r1.x), ry = fixed_to_f32(r1.y), rz = fixed_to_f32(r1.z);
+        const float dd = fmaf(dx, dx, fmaf(dy, dy, dz * dz)), q1 = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
+        const float b1 = fmaf(rx, dx, fmaf(ry, dy, rz * dz)), a0 = b1 - dd;
+        const float t = fminf(dd, q1) > kSureMin ? kSure2 * dd * (q1 + dd) : __int_as_float(0x7f800000);
+        if (a0 > 0.f && a0 * a0 > t) {
+            if (pend) approach_ended(sa, sb, i, dt);
+        } else {
+            const bool in = b1 < 0.f && b1 * b1 > t;
+            if (in && (pend || q1 * kSureUp < q)) {
+                pend = true;
+                tie = 0;
+                q = q1;
+            } else if (in ? q1 * kSureDown <= q : (pend || could_improve(q1, fmaf(-2.f, b1, q1 + dd), dd))) {
+                const I3 v2 = {2 * (a.wx - b.wx) + (A.x - B.x), 2 * (a.wy - b.wy) + (A.y - B.y),
+                               2 * (a.wz - b.wz) + (A.z - B.z)};
+                const int got = segment64(r1, d, v2, i, dt, unit(), pend, r, &tie);
+                if (got == kSegAtR0) approach_ended(sa, sb, i, dt);
+                pend = false;
+                set_q();
+            }
+        }
+        a.wx += A.x; a.wy += A.y; a.wz += A.z;
+        b.wx += B.x; b.wy += B.y; b.wz += B.z;
+    }
+    // the pending record at the start of step i (the orbits have moved on by sa, sb)
+    __device__ __forceinline__ void approach_ended(const I3 &sa, const I3 &sb, int i, double dt) {
+        Orbit32 a0 = a, b0 = b;
+        a0.x -= sa.x; a0.y -= sa.y; a0.z -= sa.z;
+        b0.x -= sb.x; b0.y -= sb.y; b0.z -= sb.z;
+        r = vertex64(a0, b0, K, s, i - 1, dt);
+        pend = false;
+        set_q();
+    }
+    // whether a segment between squared distances q0 and q1 can come nearer than the best: no point of it is nearer
+    // than the nearer end less its length
+    __device__ __forceinline__ bool could_improve(float q1, float q0, float dd) const {
+        const float m = fmaxf(fminf(fmaf(-0x1p-18f, q1 + dd, q0), q1), 0.f);
+        const float lb = sqrtf(m) * kSureDown - sqrtf(dd) * kSureUp;
+        return !(fminf(dd, q1) > kSureMin && lb > 0.f && lb * lb * kSureDown > q);
+    }
+    // after the last step: the approach may still be on
+    __device__ __forceinline__ void finish(int steps, double dt) {
+        if (pend) r = vertex64(a, b, K, s, steps, dt);
+        tie = min(tie, steps);
+    }
+    // the steps the FP64 trace takes for this clone's record (0: none, the record stands)
+    __device__ __forceinline__ int fp64_steps(int steps) const { return ok ? tie : max(steps, 1); }
+};
+
+// The clones of a warp that take the FP64 trace: n steps of each lane's clone (0: none; every lane calls).  A few are
+// traced by the whole warp one after the other, more (a step length or a reach outside the FP32 orbit's) lane by lane:
+// 4 x 32 instructions against 136.
+__device__ __forceinline__ void trace_fp64(const double *ps, int n, int steps, double dt, Approach &r) {
+    const unsigned all = 0xffffffffu;
+    unsigned m = __ballot_sync(all, n > 0);
+    if (__popc(m) > 4) {
+        if (n > 0) r = trace_clone64(ps, min(n, steps), dt);
+        return;
+    }
+    for (; m; m &= m - 1u) {
+        const int l = __ffs(m) - 1;
+        const unsigned long long p = __shfl_sync(all, (unsigned long long)ps, l);
+        const Approach x = trace_clone64_warp((const double *)p, __shfl_sync(all, min(n, steps), l),
+                                              __shfl_sync(all, dt, l));
+        if ((int)(threadIdx.x & 31) == l) r = x;
+    }
+}
+
+// a lane's clone (every lane of the warp calls; active: it has one)
+__device__ __forceinline__ Approach trace_clone(bool active, const double *__restrict__ ps, int steps, double dt) {
+    Clone32 c;
+    c.ok = c.pend = false;
+    c.tie = 0;
+    if (active && c.start(ps, steps, dt)) {
+#pragma unroll 1
+        for (int i = 1; i <= steps; i++) c.step(i, dt);
+    }
+    if (active && c.ok) c.finish(steps, dt);
+    __syncwarp();
+    trace_fp64(ps, active ? c.fp64_steps(steps) : 0, steps, dt, c.r);
+    return c.r;
 }
 
 // ---- reduction of one pair (m clones) ---------------------------------------------------------------------------
@@ -387,13 +641,12 @@ __global__ void __launch_bounds__(kMcThreads) k_pair_mc(McPairs P) {
         if (q >= P.n_items) break;
         const int4 it = P.items[q];   // x = pair, y = first clone, z = count
         const int p = it.x;
+        const int c = it.y + lane;
+        const Approach r = trace_clone(lane < it.z, P.ps + (size_t)c * 12, P.steps[p], P.dt[p]);
         if (lane < it.z) {
-            const int c = it.y + lane;
-            double best, tbest, vbest;
-            trace_clone(P.ps + (size_t)c * 12, P.steps[p], P.dt[p], best, tbest, vbest);
-            P.cres[c] = best;
-            P.cres[P.n_clones + c] = tbest;
-            P.cres[2 * (size_t)P.n_clones + c] = vbest;
+            P.cres[c] = r.best;
+            P.cres[P.n_clones + c] = r.tbest;
+            P.cres[2 * (size_t)P.n_clones + c] = r.vbest;
         }
         __threadfence();
         __syncwarp();
@@ -413,12 +666,12 @@ __global__ void __launch_bounds__(kMcThreads) k_pair_mc(McPairs P) {
 
 // Persistent clone tracing for batches replayed from a captured graph: parameters read from device memory, and the
 // launch shape a template: WARPS warps per block, CPL clones per lane traced in lockstep (items of up to 32 * CPL
-// clones; a lane past its item's end repeats its first clone and discards the copy), and MINB resident blocks per SM
+// clones; a lane past its item's end repeats another clone and discards the copy), and MINB resident blocks per SM
 // asked of the compiler (fewer registers per thread, more warps to hide the FP64 pipe's latency).  Tracing only -- the pairs are
 // reduced by k_pair_reduce_dev afterwards, which keeps this kernel's registers to the orbits'.  The clones'
 // arithmetic is the same in every variant, so every variant gives the same bits.
 template <int WARPS, int CPL, int MINB>
-__global__ void __launch_bounds__(WARPS * 32, MINB) k_pair_mc_t(const McPairs *__restrict__ Pd) {
+__global__ void __launch_bounds__(WARPS * 32, MINB > 1 ? MINB : 16 / (WARPS * CPL)) k_pair_mc_t(const McPairs *__restrict__ Pd) {
     const McPairs P = *Pd;
     const int lane = threadIdx.x & 31;
     for (;;) {
@@ -427,28 +680,34 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) k_pair_mc_t(const McPairs *_
         q = __shfl_sync(0xffffffffu, q, 0);
         if (q >= P.n_items) break;
         const int4 it = P.items[q];   // x = pair, y = first clone, z = count
-        if (lane >= it.z) continue;
         const int p = it.x;
         const int steps = P.steps[p];
-        const double dt = P.dt[p], h = 0.5 * dt;
-        Clone c[CPL];
+        const double dt = P.dt[p];
+        Clone32 c[CPL];
+        bool any = false;
 #pragma unroll
         for (int j = 0; j < CPL; j++) {
-            const int e = lane + 32 * j < it.z ? lane + 32 * j : lane;
-            c[j].start(P.ps + (size_t)(it.y + e) * 12);
+            const int e = lane + 32 * j < it.z ? lane + 32 * j : min(lane, it.z - 1);
+            any |= c[j].start(P.ps + (size_t)(it.y + e) * 12, steps, dt);
         }
+        if (any) {
 #pragma unroll 1
-        for (int i = 1; i <= steps; i++) {
+            for (int i = 1; i <= steps; i++) {
 #pragma unroll
-            for (int j = 0; j < CPL; j++) c[j].step(i, dt, h);
+                for (int j = 0; j < CPL; j++) c[j].step(i, dt);
+            }
         }
 #pragma unroll
         for (int j = 0; j < CPL; j++) {
-            if (lane + 32 * j >= it.z) continue;
-            const int cc = it.y + lane + 32 * j;
-            P.cres[cc] = c[j].best;
-            P.cres[P.n_clones + cc] = c[j].tbest;
-            P.cres[2 * (size_t)P.n_clones + cc] = c[j].vbest;
+            const bool mine = lane + 32 * j < it.z;
+            const int cc = it.y + (mine ? lane + 32 * j : 0);
+            if (c[j].ok) c[j].finish(steps, dt);
+            __syncwarp();
+            trace_fp64(P.ps + (size_t)cc * 12, mine ? c[j].fp64_steps(steps) : 0, steps, dt, c[j].r);
+            if (!mine) continue;
+            P.cres[cc] = c[j].r.best;
+            P.cres[P.n_clones + cc] = c[j].r.tbest;
+            P.cres[2 * (size_t)P.n_clones + cc] = c[j].r.vbest;
         }
     }
 }
@@ -738,17 +997,16 @@ __global__ void __launch_bounds__(kMcThreads) k_pair_mc_noalloc(int n_pairs, int
         q = __shfl_sync(0xffffffffu, q, 0);
         if (q >= n_chunks) break;
         const int c = q * 32 + lane;
+        int lo = 0, hi = n_pairs;              // clone_off[lo] <= c < clone_off[hi]
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (clone_off[mid] <= c) lo = mid; else hi = mid;
+        }
+        const Approach r = trace_clone(c < n_clones, ps + (size_t)c * 12, steps[lo], dt[lo]);
         if (c < n_clones) {
-            int lo = 0, hi = n_pairs;          // clone_off[lo] <= c < clone_off[hi]
-            while (hi - lo > 1) {
-                const int mid = (lo + hi) >> 1;
-                if (clone_off[mid] <= c) lo = mid; else hi = mid;
-            }
-            double b, t, v;
-            trace_clone(ps + (size_t)c * 12, steps[lo], dt[lo], b, t, v);
-            cres[c] = b;
-            cres[kNoAllocMaxClones + c] = t;
-            cres[2 * (size_t)kNoAllocMaxClones + c] = v;
+            cres[c] = r.best;
+            cres[kNoAllocMaxClones + c] = r.tbest;
+            cres[2 * (size_t)kNoAllocMaxClones + c] = r.vbest;
         }
     }
 }
@@ -880,6 +1138,7 @@ int orbit_setup(int dev) {
     std::memcpy(&b2, &kTinyR2, 8);
     if (b1 != kHaloCutBits || b2 != kTinyR2Bits) return 3;
     k_halo_tables<<<1, kHaloTableThreads>>>();
+    k_halo32_table<<<(kHalo32N + 255) / 256, 256>>>();
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
     if (e != cudaSuccess) return 2;
