@@ -206,10 +206,7 @@ int run_lin(PgxContext *ctx, cudaStream_t st, int N, const double *d_ps0, const 
             int nmax, Buf &opos, Buf &ovel, double *t64, float4 *t32, float *lm, bool timed, int orbit_blocks = 0) {
     RET(ensure(ctx, opos, (size_t)nmax * 21 * N * sizeof(double)));
     RET(ensure(ctx, ovel, (size_t)nmax * 3 * N * sizeof(double)));
-    int g = (int)((7L * N + 127) / 128);
-    if (orbit_blocks > 0) g = std::min(g, orbit_blocks);
-    pgx::k_stm_orbits<<<g, 128, 0, st>>>(N, d_ps0, d_npts, nmax, P<double>(opos), P<double>(ovel));
-    CKL();
+    CK(pgx::launch_stm_orbits(st, ctx->sms, N, d_ps0, d_npts, nmax, P<double>(opos), P<double>(ovel), orbit_blocks));
     if (timed) CK(cudaEventRecord(ctx->ev[EV_ORBIT], st));
     const size_t work = (size_t)N * nmax;
     pgx::k_stm_cov<<<(unsigned)((work + 255) / 256), 256, 0, st>>>(N, nmax, d_npts, P<double>(opos),

@@ -153,56 +153,66 @@ struct Orbit {
 // there are fewer orbits than the schedulers can use lanes, an orbit's independent operations go side by side: lane 0
 // holds x and the bulge, lane 1 y and the disk, lane 2 z and the halo, lane 3 the halo's side products.  A product is
 // issued as fma(a, b, -0.0), which rounds the same.  q: the lane's coordinate (lane 3: anything finite).
+// The chains are written as C_k = fma(C_k-1, X_k, Y_k) with X_k and Y_k picked by lane beforehand: a pick between two FP64
+// instructions that depend on one another would lengthen the step by its latency.
+PGX_HD constexpr double halo_coef(int n) {                                     // g_halo_coef's values
+    double c = 1.0;
+    for (int k = 0; k < n; k++) c = c * ((kHaloG1 - 1.0) - (double)k) / (double)(k + 1);
+    return c;
+}
 __device__ __forceinline__ double quad_accel(double q, int role) {
     const unsigned all = 0xffffffffu;
     const double x = __shfl_sync(all, q, 0, 4), y = __shfl_sync(all, q, 1, 4), z = __shfl_sync(all, q, 2, 4);
-    const bool bulge = role == 0, disk = role == 1, halo = role == 2;
+    const bool bulge = role == 0, disk = role == 1, halo = role == 2, help = role == 3;
+    constexpr double c0 = halo_coef(0), c1 = halo_coef(1), c2 = halo_coef(2), c3 = halo_coef(3), c4 = halo_coef(4);
+    static_assert(kPowTerms == 4, "the series below has four terms");
     const double R2 = fma(x, x, y * y);
     const double w = fma(z, z, disk ? kDiskB2 : R2);                      // r2, or z^2 + b^2 of the disk
     const double arg = w + (bulge ? kBulgeB2 : 0.0);
     const uint32_t hi = f64_hi(arg);
     bool ok = seed_ok(hi) && (disk || __double_as_longlong(w) > kTinyR2Bits);
     const double inv = rsqrt_refine(arg, widen_seed(rsqrtf(seed_arg(hi))));        // ib, iz, ir, ir
+    const double iz = __shfl_sync(all, inv, 1, 4);
     // -GM ib | a + sqrt(z^2 + b^2) | r | r, then ib^2 | D^2 | r / 12 | r / 12
-    const double A = fma(bulge ? -kBulgeGM : w, inv, disk ? kDiskA : -0.0);
+    const double A = fma(inv, bulge ? -kBulgeGM : w, disk ? kDiskA : -0.0);
+    const double gb = __shfl_sync(all, A, 0, 4);
     const double Ac = disk || __double_as_longlong(A) < kHaloCutBits ? A : kHaloCut;
     const double B = fma(bulge ? inv : Ac, bulge ? inv : (disk ? A : kHaloInvA), disk ? R2 : -0.0);
+    const double ib2 = __shfl_sync(all, B, 0, 4);
     // the halo's table entries (lanes 2 and 3), the disk's second seed
-    const long long bits = __double_as_longlong(B);
-    int e = (int)((bits >> 52) & 0x7ff) - 1023;
-    e = e < -kPow2Bias ? -kPow2Bias : (e > kPow2N - 1 - kPow2Bias ? kPow2N - 1 - kPow2Bias : e);
-    const int j = (int)((bits >> (52 - kPowSubLog)) & (kPowSub - 1));
-    const double m = __longlong_as_double((bits & 0x000fffffffffffffLL) | 0x3ff0000000000000LL);
     const uint32_t hB = f64_hi(B);
+    const int j = (int)((hB >> (20 - kPowSubLog)) & (kPowSub - 1));
+    const double invc = __ldg(&g_halo_invc[j]), powc = __ldg(&g_halo_powc[j]);
+    int e = (int)((hB >> 20) & 0x7ff) - 1023;
+    e = e < -kPow2Bias ? -kPow2Bias : (e > kPow2N - 1 - kPow2Bias ? kPow2N - 1 - kPow2Bias : e);
+    const double pow2 = __ldg(&g_halo_pow2[e + kPow2Bias]);
+    const double m = __hiloint2double((int)((hB & 0xfffffu) | 0x3ff00000u), __double2loint(B));
     ok = ok && (!disk || seed_ok(hB));
     const double yD = widen_seed(rsqrtf(seed_arg(hB)));
-    static_assert(kPowTerms == 4, "the series below has four terms");
-    //                          disk: 1 / D           halo: (1 + t)^a       helper: ir^3, -GM r / 12, c_j^a 2^(a e)
-    const double C1 = fma(disk ? yD : (halo ? m : inv), disk ? yD : (halo ? __ldg(&g_halo_invc[j]) : inv),
-                          halo ? -1.0 : -0.0);
-    const double t = C1;
-    const double C2 = fma(disk ? -B : (halo ? __ldg(&g_halo_coef[4]) : C1), disk || halo ? C1 : inv,
-                          disk ? 1.0 : (halo ? __ldg(&g_halo_coef[3]) : -0.0));
-    const double C3 = fma(disk || halo ? C2 : -kHaloGM, disk ? 0.375 : (halo ? t : B),
-                          disk ? 0.5 : (halo ? __ldg(&g_halo_coef[2]) : -0.0));
-    const double C4 = fma(disk ? C2 : (halo ? C3 : __ldg(&g_halo_pow2[e + kPow2Bias])),
-                          disk ? C3 : (halo ? t : __ldg(&g_halo_powc[j])), halo ? __ldg(&g_halo_coef[1]) : -0.0);
-    const double C5 = fma(disk ? yD : C4, disk ? C4 : t, disk ? yD : __ldg(&g_halo_coef[0]));
-    const double ir3 = __shfl_sync(all, C2, 3, 4), gx = __shfl_sync(all, C3, 3, 4), pw = __shfl_sync(all, C4, 3, 4);
-    const double C6 = (disk ? C5 : pw) * C5;                              // iD^2 | x^a
-    const double C7 = (disk ? C5 : B) * C6;                               // iD^3 | p
-    const double C8 = fma(disk ? -kDiskGM : 1.0, C7, disk ? -0.0 : 1.0);  // fd   | 1 + p
+    //                 disk: 1 / D     halo: x^a, 1 / (1 + p)     helper: ir^2, ir^3, -GM r / 12, c_j^a 2^(a e)
+    const double C1 = fma(disk ? yD : (halo ? m : inv), disk ? yD : (halo ? invc : inv), halo ? -1.0 : -0.0);
+    const double C2 = fma(C1, disk ? -B : (halo ? c4 : inv), disk ? 1.0 : (halo ? c3 : -0.0));
+    const double ir3 = __shfl_sync(all, C2, 3, 4);
+    const double C3 = fma(help ? B : C2, disk ? 0.375 : (halo ? C1 : -kHaloGM), disk ? 0.5 : (halo ? c2 : -0.0));
+    const double gx = __shfl_sync(all, C3, 3, 4);
+    const double C4 = fma(help ? powc : C3, disk ? C2 : (halo ? C1 : pow2), halo ? c1 : -0.0);
+    const double pw = __shfl_sync(all, C4, 3, 4);
+    const double C5 = fma(C4, disk ? yD : C1, disk ? yD : c0);
+    const double C6 = C5 * (disk ? C5 : pw);                              // iD^2 | x^a
+    const double C7 = C6 * (disk ? C5 : B);                               // iD^3 | p
+    const double C8 = fma(C7, disk ? -kDiskGM : 1.0, disk ? -0.0 : 1.0);  // fd   | 1 + p
+    const double fd = __shfl_sync(all, C8, 1, 4);
     const uint32_t h8 = f64_hi(C8);
     ok = ok && (!halo || seed_ok(h8));
     const double y8 = widen_seed(__frcp_rn(seed_arg(h8)));
-    const double C9 = fma(disk ? C8 : -C8, disk ? kDiskA : y8, disk ? -0.0 : 1.0);       // fd a | e
-    const double q8 = C7 * fma(y8, fma(C9, C9, C9), y8);                  // p / (1 + p)
+    const bool redo = __any_sync(all, !ok && !help);                      // an argument outside the seeds' range
+    const double C9 = fma(C8, disk ? kDiskA : -y8, disk ? -0.0 : 1.0);    // fd a | e
+    const double fda = __shfl_sync(all, C9, 1, 4);
+    const double q8 = C7 * fma(fma(C9, C9, C9), y8, y8);                  // p / (1 + p)
     const double fh = __shfl_sync(all, (gx * q8) * ir3, 2, 4);
-    const double fr = fma(__shfl_sync(all, A, 0, 4), __shfl_sync(all, B, 0, 4), fh);
-    const double g = fr + __shfl_sync(all, C8, 1, 4);
-    const double gz = fma(__shfl_sync(all, C9, 1, 4), __shfl_sync(all, inv, 1, 4), g);
-    double a = (halo ? gz : g) * q;
-    if (__any_sync(all, !ok && role != 3)) {                              // an argument outside the seeds' range
+    const double g = fma(gb, ib2, fh) + fd;
+    double a = q * (halo ? fma(fda, iz, g) : g);
+    if (redo) {
         double ax, ay, az;
         mw_accel(x, y, z, ax, ay, az);
         a = bulge ? ax : (disk ? ay : az);

@@ -80,7 +80,10 @@ struct ScreenRowDev {                // layout-identical to PgxScreenRow (includ
 int orbit_setup(int dev);
 
 // ---- kernels ------------------------------------------------------------------------------------------------------
-__global__ void k_stm_orbits(int N, const double *ps0, const int *npts, int nmax, double *opos, double *ovel);
+// the 7 orbits (nominal and neighbours) of N objects: opos[k][7][3][N], ovel[k][3][N] (nominal); npts nullptr: nmax
+// points each; max_blocks > 0: at most that many blocks, to leave room for other work
+cudaError_t launch_stm_orbits(cudaStream_t st, int sms, int N, const double *ps0, const int *npts, int nmax, double *opos,
+                              double *ovel, int max_blocks);
 __global__ void k_stm_cov(int N, int nmax, const int *npts, const double *opos, const double *ovel,
                           const double *sig21, double *t64, float4 *t32, float *lm);
 // the prefilter's coarse tracks: nominal orbits from ps (6 doubles per object), pos[k][3][N] for k < npts[i]
