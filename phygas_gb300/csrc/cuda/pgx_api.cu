@@ -574,31 +574,31 @@ int pgx_draw_pair_batch_gpu(PgxContext *ctx, int n_pairs, const PhTarget *t, con
         slot[q + 1] = slot[q] + n_clones[q];
     }
     const long long cap = slot[n_pairs];
-    const size_t bt = ((size_t)nt * sizeof(PhTarget) + 15) & ~(size_t)15;
-    const size_t bc = ((size_t)nc * sizeof(PhCluster) + 15) & ~(size_t)15;
-    const size_t bi = (((size_t)n_pairs * 4 + 15) & ~(size_t)15);
-    const size_t b8 = (size_t)n_pairs * 8;
-    RET(ensure(ctx, ctx->x_draw, bt + bc + 4 * bi + 2 * b8 + 64));
-    RET(ensure(ctx, ctx->x_draw_ps, (size_t)std::max(cap, 1LL) * 12 * 8 * 2));
+    auto pad = [](size_t b) { return (b + 15) & ~(size_t)15; };
+    const size_t bt = pad((size_t)nt * sizeof(PhTarget)), bc = pad((size_t)nc * sizeof(PhCluster));
+    const size_t bi = pad((size_t)(n_pairs + 1) * 4), b8 = pad((size_t)n_pairs * 8);
+    RET(ensure(ctx, ctx->x_draw, bt + bc + 5 * bi + 2 * b8 + pgx::pair_frames_bytes(n_pairs) + pad((size_t)cap * 4)));
     char *b = P<char>(ctx->x_draw);
-    PhTarget *d_t = (PhTarget *)b;
-    PhCluster *d_c = (PhCluster *)(b + bt);
-    int *d_ti = (int *)(b + bt + bc), *d_ci = (int *)((char *)d_ti + bi), *d_n = (int *)((char *)d_ci + bi);
-    int *d_m = (int *)((char *)d_n + bi);
-    uint64_t *d_seed = (uint64_t *)((char *)d_m + bi);
-    long long *d_slot = (long long *)(d_seed + n_pairs);
-    double *d_ps = P<double>(ctx->x_draw_ps), *d_out = d_ps + (size_t)std::max(cap, 1LL) * 12;
+    auto take = [&](size_t bytes) { char *p = b; b += bytes; return p; };
+    PhTarget *d_t = (PhTarget *)take(bt);
+    PhCluster *d_c = (PhCluster *)take(bc);
+    int *d_ti = (int *)take(bi), *d_ci = (int *)take(bi), *d_n = (int *)take(bi), *d_m = (int *)take(bi);
+    int *d_off = (int *)take(bi);
+    uint64_t *d_seed = (uint64_t *)take(b8);
+    long long *d_slot = (long long *)take(b8);
+    void *d_frames = take(pgx::pair_frames_bytes(n_pairs));
+    int *d_gi = (int *)take(0);
     CK(cudaMemcpyAsync(d_t, t, (size_t)nt * sizeof(PhTarget), cudaMemcpyHostToDevice, ctx->st));
     CK(cudaMemcpyAsync(d_c, c, (size_t)nc * sizeof(PhCluster), cudaMemcpyHostToDevice, ctx->st));
     CK(cudaMemcpyAsync(d_ti, ti, (size_t)n_pairs * 4, cudaMemcpyHostToDevice, ctx->st));
     CK(cudaMemcpyAsync(d_ci, ci, (size_t)n_pairs * 4, cudaMemcpyHostToDevice, ctx->st));
     CK(cudaMemcpyAsync(d_n, n_clones, (size_t)n_pairs * 4, cudaMemcpyHostToDevice, ctx->st));
-    CK(cudaMemcpyAsync(d_seed, seed.data(), b8, cudaMemcpyHostToDevice, ctx->st));
-    CK(cudaMemcpyAsync(d_slot, slot.data(), b8, cudaMemcpyHostToDevice, ctx->st));
+    CK(cudaMemcpyAsync(d_seed, seed.data(), (size_t)n_pairs * 8, cudaMemcpyHostToDevice, ctx->st));
+    CK(cudaMemcpyAsync(d_slot, slot.data(), (size_t)n_pairs * 8, cudaMemcpyHostToDevice, ctx->st));
     ctx->stats = PgxStats();
     CK(cudaEventRecord(ctx->ev[EV_PAIR0], ctx->st));
-    MRET(pgx::draw_pairs_gpu(ctx->st, n_pairs, d_t, d_ti, d_c, d_ci, d_n, d_seed, d_slot, d_ps, d_m,
-                             ctx->mixed.err));
+    MRET(pgx::pair_streams_gpu(ctx->st, n_pairs, d_t, d_ti, d_c, d_ci, d_n, d_seed, d_slot, d_gi, d_m, d_frames,
+                               ctx->mixed.err));
     std::vector<int> m(n_pairs);
     CK(cudaMemcpyAsync(m.data(), d_m, (size_t)n_pairs * 4, cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
@@ -609,15 +609,18 @@ int pgx_draw_pair_batch_gpu(PgxContext *ctx, int n_pairs, const PhTarget *t, con
         if (off > 2147483647LL) return fail(ctx, PGX_E_LIMIT, "pgx_draw_pair_batch_gpu: more than 2^31 clones");
         clone_off[q + 1] = (int)off;
     }
-    CK(cudaMemcpyAsync(d_n, clone_off, (size_t)n_pairs * 4, cudaMemcpyHostToDevice, ctx->st));   // offsets
-    MRET(pgx::compact_pairs_gpu(ctx->st, n_pairs, d_slot, d_n, d_m, d_ps, d_out, ctx->mixed.err));
+    RET(ensure(ctx, ctx->x_draw_ps, (size_t)std::max(off, 1LL) * 12 * 8));
+    double *d_out = P<double>(ctx->x_draw_ps);
+    CK(cudaMemcpyAsync(d_off, clone_off, (size_t)(n_pairs + 1) * 4, cudaMemcpyHostToDevice, ctx->st));
+    MRET(pgx::draw_pairs_gpu(ctx->st, n_pairs, (int)off, d_t, d_ti, d_c, d_ci, d_seed, d_slot, d_off, d_gi, d_frames,
+                             d_out, ctx->mixed.err));
     CK(cudaEventRecord(ctx->ev[EV_PAIR1], ctx->st));
     if (off > 0) CK(cudaMemcpyAsync(ps, d_out, (size_t)off * 12 * 8, cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
     ctx->stats.ms_total = elapsed(ctx, EV_PAIR0, EV_PAIR1);
     ctx->stats.clones = off;
     ctx->stats.pairs = n_pairs;
-    ctx->stats.kernels = 1;
+    ctx->stats.kernels = 2;
     return 0;
 }
 

@@ -12,8 +12,13 @@
 // (retries of non-physical draws included), so the same draws are taken.
 //   k_draw_targets   one thread per object: its nominal state and its n_samp draws in turn (the stream is
 //                    sequential: a retried draw shifts every later one), the covariance summed in the host's order
-//   k_draw_pairs     one thread per pair: its clones in turn, target then cluster per clone, into the pair's slot
-//   k_compact_pairs  the pairs' successful clones back to back (a warp per pair)
+//   k_pair_streams   one warp per pair: where in the pair's stream each of its clones begins.  A clone takes eight
+//                    Gaussians (target and cluster: parallax or distance, two proper motions, radial velocity) and one
+//                    more for each parallax or distance drawn again, so 32 clones' places are known once none of
+//                    their first tries fails; a try can fail only when its uniform deviate is below a bound
+//   k_draw_pairs     one thread per clone, from its place in the stream, into its place among the successful clones
+// One thread per pair, its clones in turn, left the GPU empty: the call for 300 pairs x 1,000 clones took 49.1 ms, by
+// clone 1.9 ms, most of it the copy of the clones to the host.
 #include <cstdint>
 #include "pgx_internal.cuh"
 #include "pgx_mixed.h"
@@ -86,18 +91,20 @@ __device__ D3 accel_ref(D3 q) {
     return add(a, mul(q, -enc / (rr * rr * rr)));
 }
 
-struct Astro { double ra, dec, plx, pmra, pmdec, rv; };
+struct Astro { double plx, pmra, pmdec, rv; };
+struct Frame { D3 r, a, d; };    // unit vectors of the line of sight, right ascension and declination
+__device__ Frame frame_of(double ra_deg, double dec_deg) {
+    const double ra = ra_deg * kRad, dec = dec_deg * kRad;
+    return Frame{d3(cos(dec) * cos(ra), cos(dec) * sin(ra), sin(dec)), d3(-sin(ra), cos(ra), 0.0),
+                 d3(-sin(dec) * cos(ra), -sin(dec) * sin(ra), cos(dec))};
+}
 
-__device__ void galcen(const Astro &a, D3 &pos, D3 &vel) {
-    const double ra = a.ra * kRad, dec = a.dec * kRad;
+__device__ void galcen(const Frame &f, const Astro &a, D3 &pos, D3 &vel) {
     const double d_kpc = 1.0 / a.plx, d_pc = d_kpc * 1000.0;
-    const D3 e_r = d3(cos(dec) * cos(ra), cos(dec) * sin(ra), sin(dec));
-    const D3 e_a = d3(-sin(ra), cos(ra), 0.0);
-    const D3 e_d = d3(-sin(dec) * cos(ra), -sin(dec) * sin(ra), cos(dec));
-    const D3 g = icrs_to_gal(mul(e_r, d_kpc));
+    const D3 g = icrs_to_gal(mul(f.r, d_kpc));
     pos = d3(g.x - kR0, g.y, g.z + kZ0);
     const double va = kAuYr * 1e-3 * a.pmra * d_pc, vd = kAuYr * 1e-3 * a.pmdec * d_pc;
-    const D3 v = add(add(mul(e_r, a.rv), mul(e_a, va)), mul(e_d, vd));
+    const D3 v = add(add(mul(f.r, a.rv), mul(f.a, va)), mul(f.d, vd));
     const D3 gv = icrs_to_gal(d3(v.x / kKmsKpcMyr, v.y / kKmsKpcMyr, v.z / kKmsKpcMyr));
     vel = add(gv, d3(kUpec / kKmsKpcMyr, (kVc + kVpec) / kKmsKpcMyr, kWpec / kKmsKpcMyr));
 }
@@ -115,64 +122,74 @@ __device__ double rv_rotation(D3 q) {
     return dot(sub(v, sun_vel()), mul(los, 1.0 / n)) * kKmsKpcMyr;
 }
 
-__device__ void close_draw(Astro a, int has_rv, double rv, double e_rv, double prior, Rng *g, double *out) {
+__device__ void close_draw(const Frame &f, Astro a, int has_rv, double rv, double e_rv, double prior, Rng *g,
+                           double *out) {
     D3 p, v;
     if (has_rv) {
         a.rv = rv + e_rv * g_or_zero(g);
     } else {
         a.rv = 0.0;
-        galcen(a, p, v);
+        galcen(f, a, p, v);
         a.rv = rv_rotation(p) + prior * g_or_zero(g);
     }
-    galcen(a, p, v);
+    galcen(f, a, p, v);
     out[0] = p.x; out[1] = p.y; out[2] = p.z; out[3] = v.x; out[4] = v.y; out[5] = v.z;
 }
 
-__device__ int sample_target(const PhTarget &t, Rng *g, double *out) {
+constexpr int kTries = 50;       // of a parallax or a distance that must be positive
+
+__device__ __forceinline__ double target_plx(const PhTarget &t, double z) {
+    return t.plx > 0 ? t.plx + t.e_plx * z : 1000.0 / (t.dist_pc * exp(t.e_lndist * z));
+}
+__device__ __forceinline__ double cluster_dist(const PhCluster &c, double z) { return c.dist_pc + c.e_dist_pc * z; }
+
+__device__ int sample_target(const PhTarget &t, const Frame &f, Rng *g, double *out) {
     Astro a;
-    a.ra = t.ra; a.dec = t.dec;
-    for (int tries = 0; tries < 50; tries++) {
-        const double plx = t.plx > 0 ? t.plx + t.e_plx * g_or_zero(g)
-                                     : 1000.0 / (t.dist_pc * exp(t.e_lndist * g_or_zero(g)));
+    for (int tries = 0; tries < kTries; tries++) {
+        const double plx = target_plx(t, g_or_zero(g));
         if (!(plx > 0)) continue;
         a.plx = plx;
         a.pmra = t.pmra + t.e_pmra * g_or_zero(g);
         a.pmdec = t.pmdec + t.e_pmdec * g_or_zero(g);
-        close_draw(a, t.has_rv, t.rv, t.e_rv, t.kind == 'P' ? PH_PULSAR_RV_PRIOR : PH_STAR_RV_PRIOR, g, out);
+        close_draw(f, a, t.has_rv, t.rv, t.e_rv, t.kind == 'P' ? PH_PULSAR_RV_PRIOR : PH_STAR_RV_PRIOR, g, out);
         return 0;
     }
     return -1;
 }
 
-__device__ int sample_cluster(const PhCluster &c, Rng *g, double *out) {
+__device__ int sample_cluster(const PhCluster &c, const Frame &f, Rng *g, double *out) {
     Astro a;
-    a.ra = c.ra; a.dec = c.dec;
-    for (int tries = 0; tries < 50; tries++) {
-        const double d = c.dist_pc + c.e_dist_pc * g_or_zero(g);
+    for (int tries = 0; tries < kTries; tries++) {
+        const double d = cluster_dist(c, g_or_zero(g));
         if (!(d > 0)) continue;
         a.plx = 1000.0 / d;
         a.pmra = c.pmra + c.e_pmra * g_or_zero(g);
         a.pmdec = c.pmdec + c.e_pmdec * g_or_zero(g);
-        close_draw(a, c.has_rv, c.rv, c.e_rv, PH_CLUSTER_RV_PRIOR, g, out);
+        close_draw(f, a, c.has_rv, c.rv, c.e_rv, PH_CLUSTER_RV_PRIOR, g, out);
         return 0;
     }
     return -1;
 }
 
-__device__ __forceinline__ int sample(const PhTarget &t, Rng *g, double *out) { return sample_target(t, g, out); }
-__device__ __forceinline__ int sample(const PhCluster &c, Rng *g, double *out) { return sample_cluster(c, g, out); }
+__device__ __forceinline__ int sample(const PhTarget &t, const Frame &f, Rng *g, double *out) {
+    return sample_target(t, f, g, out);
+}
+__device__ __forceinline__ int sample(const PhCluster &c, const Frame &f, Rng *g, double *out) {
+    return sample_cluster(c, f, g, out);
+}
 
 // nominal state and covariance of an object's draws: the covariance summed over the successful draws in draw order,
 // entry by entry, then divided by their number (the host's nominal_and_cov)
 template <class Obj>
 __device__ void object_init(const Obj &o, int n_samp, uint64_t seed, double *ps0, double *sig) {
     double nom[6], d[6], S[36];
-    sample(o, nullptr, nom);
+    const Frame f = frame_of(o.ra, o.dec);
+    sample(o, f, nullptr, nom);
     for (int q = 0; q < 36; q++) S[q] = 0.0;
     Rng g{seed};
     int k = 0;
     for (int i = 0; i < n_samp; i++) {
-        if (sample(o, &g, d)) continue;
+        if (sample(o, f, &g, d)) continue;
         const double e[6] = {d[0] - nom[0], d[1] - nom[1], d[2] - nom[2], d[3] - nom[3], d[4] - nom[4], d[5] - nom[5]};
         for (int a = 0; a < 6; a++)
             for (int b = 0; b < 6; b++) S[6 * a + b] += e[a] * e[b];
@@ -195,42 +212,103 @@ __global__ void k_draw_clusters(int n, const PhCluster *__restrict__ c, int n_sa
         object_init(c[i], n_samp, seed[i], ps0 + 6 * (size_t)i, sig + 36 * (size_t)i);
 }
 
-// ph_pair_draw for pair q: its clones at slot[q] (room for n_clones[q]), the successful ones back to back; m[q]
-__global__ void k_draw_pairs(int n_pairs, const PhTarget *__restrict__ t, const int *__restrict__ ti,
-                             const PhCluster *__restrict__ c, const int *__restrict__ ci,
-                             const int *__restrict__ n_clones, const uint64_t *__restrict__ seed,
-                             const long long *__restrict__ slot, double *__restrict__ ps, int *__restrict__ m) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= n_pairs) return;
-    const PhTarget tq = t[ti[q]];
-    const PhCluster cq = c[ci[q]];
-    Rng g{seed[q]};
-    double *o = ps + 12 * slot[q];
-    int k = 0;
-    for (int j = 0; j < n_clones[q]; j++) {
-        if (sample_target(tq, &g, o + 12 * (size_t)k) || sample_cluster(cq, &g, o + 12 * (size_t)k + 6)) continue;
-        k++;
-    }
-    m[q] = k;
+// what a pair's clones share: the frames of its target and cluster
+struct PairFrames {
+    Frame f[2];
+};
+
+// The uniform deviate from which on the first try of value + e z > 0 cannot fail: |z| <= sqrt(-2 ln u) < value / e.  The
+// margin covers every rounding; 2 = each try has to be computed (NaN included), 0 = none can fail (z is below 9.5).
+__device__ double safe_u(double value, double e) {
+    const double r = value / fabs(e) * (1.0 - 1e-9);
+    if (value > 0 && e == 0) return 0.0;
+    return r > 9.5 ? 0.0 : (r > 0 ? exp(-0.5 * r * r) * (1.0 + 1e-9) : 2.0);
 }
 
-// the successful clones of pair q (m[q] of them at slot[q]) moved to off[q], one warp per pair
-__global__ void k_compact_pairs(int n_pairs, const long long *__restrict__ slot, const int *__restrict__ off,
-                                const int *__restrict__ m, const double *__restrict__ src, double *__restrict__ dst) {
+// Where the clones of pair q begin in its stream: gi[slot[q] + k] = the Gaussians taken before its k-th successful clone,
+// m[q] = how many succeed of n_clones[q] (as ph_pair_draw takes them: a target or a cluster that fails all its tries
+// drops the clone).  Lane l of a warp looks at the clone l after the next one as if none before it drew again; the
+// clones before the first that does are settled together, that one is walked through, and the rest look again.
+__global__ void k_pair_streams(int n_pairs, const PhTarget *__restrict__ t, const int *__restrict__ ti,
+                               const PhCluster *__restrict__ c, const int *__restrict__ ci,
+                               const int *__restrict__ n_clones, const uint64_t *__restrict__ seed,
+                               const long long *__restrict__ slot, int *__restrict__ gi, int *__restrict__ m,
+                               PairFrames *__restrict__ frames) {
+    const unsigned all = 0xffffffffu;
     const int q = (int)(((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
-    if (q >= n_pairs) return;
-    const double *a = src + 12 * slot[q];
-    double *b = dst + 12 * (size_t)off[q];
-    for (int i = lane; i < 12 * m[q]; i += 32) b[i] = a[i];
+    if (q >= n_pairs) return;                                     // the whole warp: uniform
+    const PhTarget &tq = t[ti[q]];
+    const PhCluster &cq = c[ci[q]];
+    if (lane < 2) frames[q].f[lane] = lane ? frame_of(cq.ra, cq.dec) : frame_of(tq.ra, tq.dec);
+    // a target without a parallax has a positive distance times an exponential within FP64's range
+    const double ut = tq.plx > 0 ? safe_u(tq.plx, tq.e_plx)
+                                 : (tq.dist_pc > 1e-100 && tq.dist_pc < 1e100 && fabs(tq.e_lndist) < 10.0 ? 0.0 : 2.0);
+    const double uc = safe_u(cq.dist_pc, cq.e_dist_pc);
+    const uint64_t s = seed[q];
+    int *o = gi + slot[q];
+    const int n = n_clones[q];
+    int g0 = 0, k = 0;                                            // Gaussians taken, clones that succeeded
+    auto uniform = [&](int g) {                                   // the first deviate of Gaussian g
+        return (double)(splitmix_mix(s + (2 * (uint64_t)g + 1) * kGolden) >> 11) * (1.0 / 9007199254740992.0);
+    };
+    auto gauss = [&](int g) {
+        Rng r{s + 2 * (uint64_t)g * kGolden};
+        return r.gauss();
+    };
+    for (int j = 0; j < n;) {
+        const int g = g0 + 8 * lane;
+        bool bad = false;
+        if (j + lane < n) {
+            if (uniform(g) < ut) bad = !(target_plx(tq, gauss(g)) > 0);
+            if (uniform(g + 4) < uc) bad = bad || !(cluster_dist(cq, gauss(g + 4)) > 0);
+        }
+        const unsigned again = __ballot_sync(all, bad);
+        const int good = min(again ? __ffs(again) - 1 : 32, n - j);
+        if (lane < good) o[k + lane] = g;
+        k += good;
+        j += good;
+        g0 += 8 * good;
+        if (again && j < n) {                                     // clone j, try by try (every lane alike)
+            const int start = g0;
+            int a = 0, b = 0;
+            while (a < kTries && !(target_plx(tq, gauss(g0)) > 0)) { a++; g0++; }
+            if (a < kTries) {
+                g0 += 4;
+                while (b < kTries && !(cluster_dist(cq, gauss(g0)) > 0)) { b++; g0++; }
+                if (b < kTries) {
+                    g0 += 4;
+                    if (lane == 0) o[k] = start;
+                    k++;
+                }
+            }
+            j++;
+        }
+    }
+    if (lane == 0) m[q] = k;
+}
+
+// clone i of the batch (pair q's are off[q] .. off[q + 1] - 1): its draws from its place in the pair's stream.  Bound by
+// the FP64 pipe (eight Gaussians: log, cos and sqrt each); the pair is found by bisection, the frames come precomputed.
+__global__ void __launch_bounds__(128) k_draw_pairs(int n_pairs, int n, const PhTarget *__restrict__ t,
+                                                    const int *__restrict__ ti, const PhCluster *__restrict__ c,
+                                                    const int *__restrict__ ci, const uint64_t *__restrict__ seed,
+                                                    const long long *__restrict__ slot, const int *__restrict__ off,
+                                                    const int *__restrict__ gi, const PairFrames *__restrict__ frames,
+                                                    double *__restrict__ ps) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    int q = 0, hi = n_pairs;                                      // off[q] <= i < off[hi]
+    while (hi - q > 1) {
+        const int mid = (q + hi) >> 1;
+        if (off[mid] <= i) q = mid; else hi = mid;
+    }
+    Rng g{seed[q] + 2 * (uint64_t)gi[slot[q] + (i - off[q])] * kGolden};
+    double *o = ps + 12 * (size_t)i;
+    sample_target(t[ti[q]], frames[q].f[0], &g, o);
+    sample_cluster(c[ci[q]], frames[q].f[1], &g, o + 6);
 }
 
 }  // namespace
-
-int compact_pairs_gpu(cudaStream_t st, int n_pairs, const long long *slot, const int *off, const int *m,
-                      const double *src, double *dst, std::string &err) {
-    k_compact_pairs<<<(unsigned)(((size_t)n_pairs * 32 + 255) / 256), 256, 0, st>>>(n_pairs, slot, off, m, src, dst);
-    return check(cudaGetLastError(), err, "k_compact_pairs");
-}
 
 int draw_targets_gpu(cudaStream_t st, int n, const PhTarget *t, int n_samp, const uint64_t *seed, double *ps0,
                      double *sig, std::string &err) {
@@ -244,10 +322,22 @@ int draw_clusters_gpu(cudaStream_t st, int n, const PhCluster *c, int n_samp, co
     return check(cudaGetLastError(), err, "k_draw_clusters");
 }
 
-int draw_pairs_gpu(cudaStream_t st, int n_pairs, const PhTarget *t, const int *ti, const PhCluster *c,
-                   const int *ci, const int *n_clones, const uint64_t *seed, const long long *slot, double *ps,
-                   int *m, std::string &err) {
-    k_draw_pairs<<<(n_pairs + 63) / 64, 64, 0, st>>>(n_pairs, t, ti, c, ci, n_clones, seed, slot, ps, m);
+size_t pair_frames_bytes(int n_pairs) { return (size_t)n_pairs * sizeof(PairFrames); }
+
+int pair_streams_gpu(cudaStream_t st, int n_pairs, const PhTarget *t, const int *ti, const PhCluster *c, const int *ci,
+                     const int *n_clones, const uint64_t *seed, const long long *slot, int *gi, int *m, void *frames,
+                     std::string &err) {
+    k_pair_streams<<<(unsigned)(((size_t)n_pairs * 32 + 127) / 128), 128, 0, st>>>(
+        n_pairs, t, ti, c, ci, n_clones, seed, slot, gi, m, static_cast<PairFrames *>(frames));
+    return check(cudaGetLastError(), err, "k_pair_streams");
+}
+
+int draw_pairs_gpu(cudaStream_t st, int n_pairs, int n, const PhTarget *t, const int *ti, const PhCluster *c,
+                   const int *ci, const uint64_t *seed, const long long *slot, const int *off, const int *gi,
+                   const void *frames, double *ps, std::string &err) {
+    if (n <= 0) return 0;
+    k_draw_pairs<<<(unsigned)(((size_t)n + 127) / 128), 128, 0, st>>>(
+        n_pairs, n, t, ti, c, ci, seed, slot, off, gi, static_cast<const PairFrames *>(frames), ps);
     return check(cudaGetLastError(), err, "k_draw_pairs");
 }
 
