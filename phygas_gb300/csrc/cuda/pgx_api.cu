@@ -389,8 +389,7 @@ int screen_slot(PgxContext *ctx, int s, double cut, int precision, long *n_rows,
                                                                      rows);
         CKL();
         if (precision == PGX_FP64) {
-            pgx::k_finish64<<<(unsigned)(((size_t)total * 32 + 255) / 256), 256, 0, ctx->st>>>(
-                total, P<pgx::FinishIn>(ctx->fin), rows);
+            pgx::launch_finish64(ctx->st, total, P<pgx::FinishIn>(ctx->fin), rows);
             CKL();
         } else {
             MRET(pgx::mixed_finish(ctx->st, total, P<pgx::FinishIn>(ctx->fin), rows, ctx->mixed, &ctx->stats));
@@ -1810,7 +1809,7 @@ int finish_one(PgxContext *ctx, const PhLin *tl, const PhLin *cl, const PhCluste
     pgx::ScreenRowDev *row = (pgx::ScreenRowDev *)(b + sizeof kp + sizeof(pgx::FinishIn));
     pgx::k_finish_prep<<<1, 32, 0, ctx->st>>>(T, 1, (const pgx::KeptPair *)b, fin, row);
     CKL();
-    pgx::k_finish64<<<1, 32, 0, ctx->st>>>(1, fin, row);
+    pgx::launch_finish64(ctx->st, 1, fin, row);
     CKL();
     pgx::ScreenRowDev r;
     CK(cudaMemcpyAsync(&r, row, sizeof r, cudaMemcpyDeviceToHost, ctx->st));

@@ -112,6 +112,6 @@ __global__ void k_exclusive_scan(int n, const int *in, int *out, int *total);
 __global__ void k_emit_kept(int nt, int nc, const double *chi2T, const int *kbT, const double *sbT, double cut,
                             const int *off, KeptPair *out);
 __global__ void k_finish_prep(ScreenTables T, int n, const KeptPair *kp, FinishIn *fin, ScreenRowDev *rows);
-__global__ void k_finish64(int n, const FinishIn *fin, ScreenRowDev *rows);
+void launch_finish64(cudaStream_t st, int n, const FinishIn *fin, ScreenRowDev *rows);
 
 }  // namespace pgx

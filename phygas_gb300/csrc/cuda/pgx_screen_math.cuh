@@ -75,6 +75,9 @@ struct ScanState {
                                           const double (&m1)[3], bool more, double cut) {
         double s;
         const double q = point_chi2_64(M, R2, m0, m1, more, cut, s);
+        fold(k, q, s);
+    }
+    __device__ __forceinline__ void fold(int k, double q, double s) {
         if (q >= 0 && q < best) { best = q; kb = k; sb = s; }
     }
 };
@@ -123,14 +126,18 @@ __device__ __forceinline__ double gauss64(uint64_t a, uint64_t b) {
 }
 
 // position of draw i of a kept pair (its Gaussians are calls 6i+1 .. 6i+6 of the pair's stream)
-__device__ __forceinline__ void draw_xyz64(const FinishIn &f, int i, double &x, double &y, double &z) {
+__device__ __forceinline__ void draw_xyz64(const FinishIn &f, int i, double z0, double &x, double &y, double &z) {
     const uint64_t n = 6ull * (uint64_t)i;
-    const double z0 = gauss64(splitmix_at(f.seed, n + 1), splitmix_at(f.seed, n + 2));
     const double z1 = gauss64(splitmix_at(f.seed, n + 3), splitmix_at(f.seed, n + 4));
     const double z2 = gauss64(splitmix_at(f.seed, n + 5), splitmix_at(f.seed, n + 6));
     x = f.mx + f.l00 * z0;
     y = f.my + f.l10 * z0 + f.l11 * z1;
     z = f.mz + f.l20 * z0 + f.l21 * z1 + f.l22 * z2;
+}
+
+__device__ __forceinline__ void draw_xyz64(const FinishIn &f, int i, double &x, double &y, double &z) {
+    const uint64_t n = 6ull * (uint64_t)i;
+    draw_xyz64(f, i, gauss64(splitmix_at(f.seed, n + 1), splitmix_at(f.seed, n + 2)), x, y, z);
 }
 
 // draw i of a kept pair: bit 0 = inside r50, bit 1 = inside rtot
