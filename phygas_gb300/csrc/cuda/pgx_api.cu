@@ -4,7 +4,8 @@
 // Stage sequence of one screen chunk (all on the context's stream, no host round trip before the kept-pair count):
 //   k_stm_orbits -> k_stm_cov -> k_scan64 -> k_count_kept -> k_exclusive_scan -> [count to host] -> k_emit_kept
 //   -> k_finish_prep -> k_finish64            (the FP64 path; the mixed path replaces scan..finish, pgx_mixed.cu)
-// Pair Monte Carlo: one persistent k_pair_mc launch over a longest-first queue (+ k_pair_reduce_big).
+// Pair Monte Carlo: one persistent trace kernel over a longest-first queue and the reductions, as a captured graph (+
+// k_pair_reduce_big).
 #include <algorithm>
 #include <chrono>
 #include <cmath>
@@ -114,7 +115,7 @@ struct PgxContext {
     pgx::MixedBufs mixed;
     long n_rows = 0;
     // pair Monte Carlo
-    Buf p_off, p_ps, p_steps, p_dt, p_r50, p_rt, p_items, p_q, p_done, p_cres, p_res, p_params;
+    Buf p_off, p_ps, p_steps, p_dt, p_r50, p_rt, p_items, p_q, p_cres, p_res, p_params;
     int mc_variant = 0;                        // launch shape of the clone kernel (pgx_tune_pair picks it)
     int mc_blocks_per_sm = 0;                  // > 0: the persistent clone kernels on at most this many blocks per SM
     const int *mc_busy = nullptr;              // set: the cap applies only while *mc_busy is nonzero at a launch
@@ -469,7 +470,7 @@ void pgx_close(PgxContext *ctx) {
                    &ctx->cname, &ctx->chi2T,
                    &ctx->kbT, &ctx->sbT, &ctx->cnt, &ctx->off, &ctx->total, &ctx->kept, &ctx->fin, &ctx->rows,
                    &ctx->p_off, &ctx->p_ps, &ctx->p_steps, &ctx->p_dt, &ctx->p_r50, &ctx->p_rt, &ctx->p_items,
-                   &ctx->p_q, &ctx->p_done, &ctx->p_cres, &ctx->p_res, &ctx->p_params, &ctx->x_ps0, &ctx->x_sig21,
+                   &ctx->p_q, &ctx->p_cres, &ctx->p_res, &ctx->p_params, &ctx->x_ps0, &ctx->x_sig21,
                    &ctx->x_npts,
                    &ctx->x_opos, &ctx->x_ovel, &ctx->x_t64, &ctx->x_t32, &ctx->rows_b[0], &ctx->rows_b[1],
                    &ctx->lab_names, &ctx->lab_kinds, &ctx->lab_age16, &ctx->lab_age84, &ctx->part_in,
@@ -1446,6 +1447,7 @@ int mc_graph(PgxContext *ctx, int v, bool capped, cudaGraphExec_t &exec) {
     return 0;
 }
 
+// variant < 0: the context's, or eight lanes per clone for few clones
 int pair_run(PgxContext *ctx, int variant, int n_pairs, const int *clone_off, const double *ps, const int *steps,
              const double *dt, const double *r50_pc, const double *rtot_pc, PhResult *res, double *clone_out) {
     if (!ctx) return PGX_E_ARG;
@@ -1455,8 +1457,6 @@ int pair_run(PgxContext *ctx, int variant, int n_pairs, const int *clone_off, co
     CK(cudaSetDevice(ctx->device));
     const int M = clone_off[n_pairs];
     if (clone_off[0] != 0 || M < 0 || (M > 0 && !ps)) return fail(ctx, PGX_E_ARG, "pgx_pair: clone_off");
-    int warps = 4, cpl = 1, minb = 1;
-    pgx::mc_variant_shape(variant, warps, cpl, minb);
     int mmax = 0;
     for (int p = 0; p < n_pairs; p++) {
         const int m = clone_off[p + 1] - clone_off[p];
@@ -1466,20 +1466,16 @@ int pair_run(PgxContext *ctx, int variant, int n_pairs, const int *clone_off, co
         if (steps[p] < 0) return fail(ctx, PGX_E_ARG, "pgx_pair: steps[%d] = %d", p, steps[p]);
         mmax = std::max(mmax, m);
     }
-    // pairs of at most 1024 clones (every batch of the benchmark and serving workloads) run the captured
-    // prep + trace + reduce graph; bigger pairs the fused kernel and the block-wide reduction
-    const bool graph = mmax <= 1024;
-    const int chunk = graph ? 32 * cpl : 32;
+    if (variant < 0) variant = M <= pgx::kMcQuadClones * ctx->sms ? pgx::mc_quad_variant() : ctx->mc_variant;
+    int warps = 4, cpl = 1, minb = 1;
+    pgx::mc_variant_shape(variant, warps, cpl, minb);
+    const int chunk = cpl > 0 ? 32 * cpl : 4;
     std::vector<int4> items;
-    int big_n2 = 0;
+    int sort_max = 0;
     long long clone_steps = 0;
     for (int p = 0; p < n_pairs; p++) {
         const int m = clone_off[p + 1] - clone_off[p];
-        if (m > 1024 && m <= pgx::kSortMax) {
-            int n2 = 1;
-            while (n2 < m) n2 <<= 1;
-            big_n2 = std::max(big_n2, n2);
-        }
+        if (m <= pgx::kSortMax) sort_max = std::max(sort_max, m);
         for (int c0 = 0; c0 < m; c0 += chunk)
             items.push_back(make_int4(p, clone_off[p] + c0, std::min(chunk, m - c0), 0));
         clone_steps += (long long)m * steps[p];
@@ -1493,7 +1489,6 @@ int pair_run(PgxContext *ctx, int variant, int n_pairs, const int *clone_off, co
     RET(ensure(ctx, ctx->p_rt, (size_t)n_pairs * 8));
     RET(ensure(ctx, ctx->p_items, items.size() * sizeof(int4)));
     RET(ensure(ctx, ctx->p_q, 16));
-    RET(ensure(ctx, ctx->p_done, (size_t)n_pairs * 4));
     RET(ensure(ctx, ctx->p_cres, (size_t)M * 3 * 8));
     RET(ensure(ctx, ctx->p_res, (size_t)n_pairs * sizeof(PhResult)));
     CK(cudaMemcpyAsync(ctx->p_off.p, clone_off, (size_t)(n_pairs + 1) * 4, cudaMemcpyHostToDevice, ctx->st));
@@ -1508,38 +1503,19 @@ int pair_run(PgxContext *ctx, int variant, int n_pairs, const int *clone_off, co
     Pp.n_pairs = n_pairs; Pp.n_clones = M; Pp.n_items = (int)items.size();
     Pp.clone_off = P<int>(ctx->p_off); Pp.ps = P<double>(ctx->p_ps); Pp.steps = P<int>(ctx->p_steps);
     Pp.dt = P<double>(ctx->p_dt); Pp.r50_pc = P<double>(ctx->p_r50); Pp.rtot_pc = P<double>(ctx->p_rt);
-    Pp.items = P<int4>(ctx->p_items); Pp.qhead = P<int>(ctx->p_q); Pp.done = P<int>(ctx->p_done);
+    Pp.items = P<int4>(ctx->p_items); Pp.qhead = P<int>(ctx->p_q);
     Pp.cres = P<double>(ctx->p_cres); Pp.res = P<pgx::PhResultDev>(ctx->p_res);
     ctx->stats = PgxStats();
-    if (graph) {
-        cudaGraphExec_t exec;
-        RET(mc_graph(ctx, variant, mc_cap_now(ctx) > 0, exec));
-        // the parameters travel by copy: the graph's kernels read them from p_params
-        CK(cudaMemcpyAsync(ctx->p_params.p, &Pp, sizeof Pp, cudaMemcpyHostToDevice, ctx->st));
-        CK(cudaEventRecord(ctx->ev[EV_PAIR0], ctx->st));
-        CK(cudaGraphLaunch(exec, ctx->st));
-        ctx->stats.kernels += 3;
-    } else {
-        CK(cudaMemsetAsync(ctx->p_q.p, 0, 16, ctx->st));
-        CK(cudaMemsetAsync(ctx->p_done.p, 0, (size_t)n_pairs * 4, ctx->st));
-        CK(cudaEventRecord(ctx->ev[EV_PAIR0], ctx->st));
-        if (!items.empty()) {
-            int per_sm = 0;
-            CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pgx::k_pair_mc, pgx::kMcThreads, 0));
-            const int warps_needed = (int)items.size();
-            int grid = std::max(1, ctx->sms * std::max(1, per_sm));
-            const int cap = mc_cap_now(ctx);
-            if (cap > 0) grid = std::min(grid, cap * ctx->sms);
-            grid = std::min(grid, (warps_needed + pgx::kMcThreads / 32 - 1) / (pgx::kMcThreads / 32));
-            pgx::k_pair_mc<<<grid, pgx::kMcThreads, 0, ctx->st>>>(Pp);
-            CKL();
-            ctx->stats.kernels++;
-        }
-        const size_t smem = (size_t)big_n2 * 8;
-        if (smem > 48 * 1024)
-            CK(cudaFuncSetAttribute(pgx::k_pair_reduce_big, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        pgx::k_pair_reduce_big<<<n_pairs, 256, smem, ctx->st>>>(Pp);
-        CKL();
+    // prep, trace and the reduction of pairs of at most 1024 clones; the parameters travel by copy: the graph's kernels
+    // read them from p_params
+    cudaGraphExec_t exec;
+    RET(mc_graph(ctx, variant, mc_cap_now(ctx) > 0, exec));
+    CK(cudaMemcpyAsync(ctx->p_params.p, &Pp, sizeof Pp, cudaMemcpyHostToDevice, ctx->st));
+    CK(cudaEventRecord(ctx->ev[EV_PAIR0], ctx->st));
+    CK(cudaGraphLaunch(exec, ctx->st));
+    ctx->stats.kernels += 3;
+    if (mmax > 1024) {
+        CK(pgx::launch_pair_reduce_big(ctx->st, Pp, sort_max));
         ctx->stats.kernels++;
     }
     CK(cudaEventRecord(ctx->ev[EV_PAIR1], ctx->st));
@@ -1560,7 +1536,7 @@ int pair_run(PgxContext *ctx, int variant, int n_pairs, const int *clone_off, co
 int pgx_pair(PgxContext *ctx, int n_pairs, const int *clone_off, const double *ps, const int *steps, const double *dt,
              const double *r50_pc, const double *rtot_pc, PhResult *res, double *clone_out) {
     if (!ctx) return PGX_E_ARG;
-    return pair_run(ctx, ctx->mc_variant, n_pairs, clone_off, ps, steps, dt, r50_pc, rtot_pc, res, clone_out);
+    return pair_run(ctx, -1, n_pairs, clone_off, ps, steps, dt, r50_pc, rtot_pc, res, clone_out);
 }
 
 int pgx_pair_targets(PgxContext *ctx, int n_pairs, const PhTarget *t, const int *ti, const PhCluster *c, const int *ci,
@@ -1615,7 +1591,7 @@ int pgx_pair_targets(PgxContext *ctx, int n_pairs, const PhTarget *t, const int 
             rc = fail(ctx, x.rc == -1 ? PGX_E_NOMEM : PGX_E_LIMIT, "pgx_pair_targets: clone draws of pairs %d..%d",
                       x.p0, x.p0 + x.n);
         } else {
-            rc = pair_run(ctx, ctx->mc_variant, x.n, x.off.data(), ctx->h_clones[i], x.steps.data(), x.dt.data(),
+            rc = pair_run(ctx, -1, x.n, x.off.data(), ctx->h_clones[i], x.steps.data(), x.dt.data(),
                           x.r50.data(), x.rt.data(), res + x.p0, nullptr);
             const PgxStats &st = ctx->stats;
             sum.ms_pair += st.ms_pair;
@@ -1843,13 +1819,7 @@ int reduce_only(PgxContext *ctx, int m, const double *best, const double *tbest,
     Pp.r50_pc = P<double>(ctx->p_r50); Pp.rtot_pc = P<double>(ctx->p_rt); Pp.res = P<pgx::PhResultDev>(ctx->p_res);
     pgx::k_pair_reduce_only<<<1, pgx::kMcThreads, 0, ctx->st>>>(Pp);
     CKL();
-    int n2 = 1;
-    while (n2 < m) n2 <<= 1;
-    const size_t smem = m > 1024 && m <= pgx::kSortMax ? (size_t)n2 * 8 : 0;
-    if (smem > 48 * 1024)
-        CK(cudaFuncSetAttribute(pgx::k_pair_reduce_big, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    pgx::k_pair_reduce_big<<<1, 256, smem, ctx->st>>>(Pp);
-    CKL();
+    CK(pgx::launch_pair_reduce_big(ctx->st, Pp, m <= pgx::kSortMax ? m : 0));
     CK(cudaMemcpyAsync(res, ctx->p_res.p, sizeof(PhResult), cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
     return 0;

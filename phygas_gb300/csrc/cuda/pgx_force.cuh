@@ -232,4 +232,38 @@ struct QuadOrbit {
     }
 };
 
+// force32 (pgx_orbit32.cuh) on four lanes per orbit, as quad_accel does it for FP64: the same operations on the same
+// operands, so the same bits, in about 270 instructions a step for 8 orbits a warp where one lane per orbit takes 340
+// for 32.  That is three times the issue slots, but a step is then some 900 cycles long for a warp alone and not 2,300:
+// for batches that leave the schedulers idle.  Lane 0 holds x and the bulge, 1 y and the disk, 2 z and the halo, 3 a
+// coordinate that stays 0.
+__device__ __forceinline__ F2 quad_shfl(F2 v, int src) {
+    return F2{__shfl_sync(0xffffffffu, v.h, src, 4), __shfl_sync(0xffffffffu, v.l, src, 4)};
+}
+__device__ __forceinline__ F2 f2_pick(bool a, F2 x, F2 y) { return F2{a ? x.h : y.h, a ? x.l : y.l}; }
+// K's constant of the lane's role (lane 3: the halo's)
+__device__ __forceinline__ F3 quad_constant(const Force32 &K, int role) {
+    return role == 0 ? K.bulge : (role == 1 ? K.disk : K.halo);
+}
+// x: the lane's coordinate; its acceleration in displacement units
+__device__ __forceinline__ int64_t quad_accel32(const F3 &k, float c, int64_t x, int role, float &r2out) {
+    using M = MwModel32;
+    const bool bulge = role == 0, disk = role == 1;
+    const F2 f = fixed_to_f2(x, c), sq = f2_sqr(f);
+    const F2 z2 = quad_shfl(sq, 2), R2 = f2_add(quad_shfl(sq, 0), quad_shfl(sq, 1)), r2 = f2_add(R2, z2);
+    r2out = r2.h;
+    const F2 u = halo32_power<M>(HaloTable32(), r2);
+    const F2 arg = f2_add(f2_pick(disk, z2, r2), bulge ? M::bulge_b2() : (disk ? M::disk_b2() : F2{0.f, 0.f}));
+    const F2 inv = f2_rsqrt(arg);                                                   // ib | iz | ir
+    const F2 a = f2_add(f2_mul(f2_pick(disk, arg, inv), f2_pick(disk, inv, u)), disk ? M::disk_a() : F2{1.f, 0.f});
+    const F2 q = f2_sqr(f2_pick(disk, a, inv));                                     // s^2 | ir^2
+    const F2 iD = f2_rsqrt(f2_add(q, R2)), rc = f2_rcp(a);
+    const F2 cube = f2_cube(f2_pick(disk, iD, inv));                                // ib^3 | D^-3 | ir^3
+    F2 e = f2_mul3(f2_pick(role >= 2, f2_mul(q, rc), cube), k);                     // bulge | disk | halo
+    if (role >= 2 && !(r2.h < M::cut2)) e = f2_mul3(f2_mul3(cube, k), M::far());
+    const F2 ez = f2_mul(e, f2_mul(a, inv));                                        // (disk) along z
+    const F2 g1 = f2_add(quad_shfl(e, 2), quad_shfl(e, 0)), fd = quad_shfl(e, 1), fz = quad_shfl(ez, 1);
+    return acc_to_fixed(f2_mul(f2_norm(f2_add(g1, f2_pick(role == 2, fz, fd))), f));
+}
+
 }  // namespace pgx

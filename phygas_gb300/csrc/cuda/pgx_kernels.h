@@ -12,6 +12,9 @@ struct PhResultDev {
 };
 
 constexpr int kMcThreads = 128;
+// Batches of at most this many clones per SM take eight lanes per clone (k_pair_mc_quad): up to two warps a scheduler.
+// 2,000 steps, one lane against eight: 1 x 1,000 clones 1.86 and 1.10 ms, 4,000 2.00 and 1.60, 10,000 2.24 and 2.72.
+constexpr int kMcQuadClones = 32, kMcQuadWarps = 4;
 
 // Clone Monte Carlo work: clones of pair p are [clone_off[p], clone_off[p+1]); ps = 12 doubles per clone
 struct McPairs {
@@ -21,9 +24,8 @@ struct McPairs {
     const int *steps;         // per pair
     const double *dt;         // per pair (negative)
     const double *r50_pc, *rtot_pc;
-    const int4 *items;        // (pair, first clone, count <= 32, -)
-    int *qhead;               // queue head (zeroed before launch)
-    int *done;                // per pair, clones finished (zeroed before launch)
+    const int4 *items;        // (pair, first clone, count, -)
+    int *qhead;               // queue head (set by k_mc_prep)
     double *cres;             // [3][n_clones]: best (kpc), tbest (Myr), vbest (kpc/Myr)
     PhResultDev *res;         // per pair
 };
@@ -88,20 +90,19 @@ __global__ void k_stm_cov(int N, int nmax, const int *npts, const double *opos, 
                           const double *sig21, double *t64, float4 *t32, float *lm);
 // the prefilter's coarse tracks: nominal orbits from ps (6 doubles per object), pos[k][3][N] for k < npts[i]
 cudaError_t launch_coarse_tracks(cudaStream_t st, int N, const double *ps, const int *npts, double *pos);
-__global__ void k_pair_mc(McPairs P);
 // launch-shape variants of the persistent clone kernel (parameters in device memory): count, shape (warps per block,
 // clones per lane), full persistent grid, and the prep + trace + reduce kernels as one sequence on a stream (pairs of
 // at most 1024 clones)
 int mc_variants();
+int mc_quad_variant();               // the variant after the tuner's: eight lanes per clone, items of 4 clones
 void mc_variant_shape(int v, int &warps, int &cpl, int &min_blocks);
 cudaError_t mc_variant_grid(int v, int sms, int &grid);
 cudaError_t launch_mc(int v, int grid, int prep_grid, int reduce_grid, cudaStream_t st, const McPairs *Pd);
-// pairs of more than 1024 clones: sorted in shared memory up to kSortMax clones (dynamic shared memory of the launch:
-// the batch's largest such pair rounded up to a power of two, times 8 bytes), beyond that reduced by radix selection
+// pairs of more than 1024 clones: sorted in shared memory up to kSortMax clones, beyond that reduced by radix selection
 constexpr int kSortMax = 16384;
 // the most clones of one pair (the clone offsets are 32-bit)
 constexpr int kMaxPairClones = 1 << 26;
-__global__ void k_pair_reduce_big(McPairs P);
+cudaError_t launch_pair_reduce_big(cudaStream_t st, const McPairs &P, int sort_max);
 __global__ void k_pair_reduce_only(McPairs P);
 __global__ void k_peak_dfma(double *out, int iters, double a, double b);
 __global__ void k_peak_ffma(float *out, int iters, float a, float b);

@@ -8,14 +8,14 @@
 //   k_stm_cov      one thread per (object, point): A = (neighbour - nominal) / eps, S = A Sigma0 A^T, and the
 //                  track layouts the screen reads (FP64 for the exact stages, split FP32 for the filter, and a
 //                  lower bound on the smallest eigenvalue of S for the filter's error bounds)
-//   k_pair_mc      persistent: warps take items of <= 32 clones of one pair from a device queue (longest first),
-//                  trace them back with KDK leapfrog and the segment closest approach (reference ph_pair_clone,
-//                  src/phygas.c:200-216), on the FP32 and integer units where they are as accurate; the warp that finishes a pair's last item reduces it in registers
-//                  with warp shuffles (reference ph_pair_reduce, src/phygas.c:218-238)
-//   k_pair_reduce_big  the same reduction for pairs of more than 1024 clones, one CTA per pair in shared memory
-//   k_mc_prep, k_pair_mc_t, k_pair_reduce_dev  the same work as one captured CUDA graph for batches of pairs of at
-//                  most 1024 clones: parameters read from device memory, tracing separate from the reduction, and
-//                  the tracing kernel's launch shape (warps per block, clones per lane) a template the autotuner picks
+//   k_mc_prep, k_pair_mc_t, k_pair_reduce_dev  the clone Monte Carlo as one captured CUDA graph, its parameters read
+//                  from device memory.  k_pair_mc_t is persistent: warps take items of clones of one pair from a device
+//                  queue (longest first) and trace them back with KDK leapfrog and the segment closest approach
+//                  (reference ph_pair_clone, src/phygas.c:200-216), on the FP32 and integer units where they are as
+//                  accurate; its launch shape (warps per block, clones per lane) is a template the autotuner picks.
+//                  k_pair_mc_quad: eight lanes per clone, for batches of few clones.  k_pair_reduce_dev: a warp per
+//                  pair reduces it in registers with warp shuffles (reference ph_pair_reduce, src/phygas.c:218-238)
+//   k_pair_reduce_big  the same reduction for pairs of more than 1024 clones, one CTA per pair
 //
 // Built with --fmad=false: every fused multiply-add is an explicit fma(), so the rounding does not depend on how the
 // compiler arranges a kernel, and every launch shape gives the same bits.
@@ -108,38 +108,6 @@ cudaError_t launch_stm_orbits(cudaStream_t st, int sms, int N, const double *ps0
         if (max_blocks > 0) g = std::min(g, (long)max_blocks);
         k_stm_orbits<<<(unsigned)g, threads, 0, st>>>(N, ps0, npts, nmax, opos, ovel);
     }
-    return cudaGetLastError();
-}
-
-// Coarse tracks of the prefilter (reference track, src/phygas.c:98-111): the nominal orbit of each object from ps
-// (6 doubles per object), one thread per object; pos[k][3][N] = the position after 10 k KDK steps of -0.05 Myr, for
-// k < npts[i].  The same orbit, steps and force as k_stm_orbits' nominal orbit.
-__global__ void __launch_bounds__(32) k_coarse_tracks(int N, const double *__restrict__ ps,
-                                                      const int *__restrict__ npts, double *__restrict__ pos) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= N) return;
-    const size_t NN = N;
-    const double *q = ps + 6 * (size_t)i;
-    Orbit o;
-    o.x = q[0]; o.y = q[1]; o.z = q[2]; o.vx = q[3]; o.vy = q[4]; o.vz = q[5];
-    o.init();
-    const int n = npts[i];
-    constexpr double dt = -kStepMyr / kSub, h = 0.5 * dt;
-    for (int k = 0; k < n; k++) {
-        if (k > 0) {
-#pragma unroll 1
-            for (int s = 0; s < kSub; s++) o.kdk(dt, h);
-        }
-        double *p = pos + (size_t)k * 3 * NN + i;
-        p[0] = o.x; p[NN] = o.y; p[2 * NN] = o.z;
-    }
-}
-
-cudaError_t launch_coarse_tracks(cudaStream_t st, int N, const double *ps, const int *npts, double *pos) {
-    if (N <= 0) return cudaSuccess;
-    // a warp per block: the few hundred to few thousand orbits spread over every SM, each warp with an SM's FP64
-    // pipe to itself
-    k_coarse_tracks<<<(N + 31) / 32, 32, 0, st>>>(N, ps, npts, pos);
     return cudaGetLastError();
 }
 
@@ -418,55 +386,99 @@ __device__ __noinline__ Approach vertex64(const Orbit32 a, const Orbit32 b, cons
                     norm64(v2) * (u * (1.0 / 128.0)) / fabs(dt)};
 }
 
+// The closest approach so far, from the float estimates of each step
+struct Near32 {
+    Approach r;
+    float q;                 // r.best^2 in squared high-word units
+    int tie;                 // > 0: the record is a tie that the FP64 trace of this many steps decides
+    bool pend;
+    __device__ __forceinline__ void set_q(const OrbitScale &s) {
+        const float f = (float)(r.best * __hiloint2double((1023 + 23 - s.e) << 20, 0));
+        q = f * f;
+    }
+    __device__ __forceinline__ void start(const double *p, const OrbitScale &s) {
+        const double rx = p[0] - p[6], ry = p[1] - p[7], rz = p[2] - p[8];
+        const double ux = p[3] - p[9], uy = p[4] - p[10], uz = p[5] - p[11];
+        r = Approach{sqrt(fma(rx, rx, fma(ry, ry, rz * rz))), 0.0, sqrt(fma(ux, ux, fma(uy, uy, uz * uz)))};
+        pend = false;
+        tie = 0;
+        set_q(s);
+    }
+    // a step's dd = d.d, q1 = r1.r1, b1 = r1.d; segment(at_r0) runs segment64 on it, vertex() the record at its start
+    template <class Segment, class Vertex>
+    __device__ __forceinline__ void step(float dd, float q1, float b1, const OrbitScale &s, const Segment &segment,
+                                         const Vertex &vertex) {
+        const float a0 = b1 - dd;
+        const float t = fminf(dd, q1) > kSureMin ? kSure2 * dd * (q1 + dd) : __int_as_float(0x7f800000);
+        if (a0 > 0.f && a0 * a0 > t) {
+            if (!pend) return;
+            r = vertex();                                     // the approach ended at r0
+        } else {
+            const bool in = b1 < 0.f && b1 * b1 > t;
+            if (in && (pend || q1 * kSureUp < q)) {
+                pend = true;
+                tie = 0;
+                q = q1;
+                return;
+            }
+            if (!(in ? q1 * kSureDown <= q : (pend || could_improve(q1, fmaf(-2.f, b1, q1 + dd), dd)))) return;
+            if (segment(pend, r, &tie) == kSegAtR0) r = vertex();
+        }
+        pend = false;
+        set_q(s);
+    }
+    // whether a segment between squared distances q0 and q1 can come nearer than the best: no point of it is nearer
+    // than the nearer end less its length
+    __device__ __forceinline__ bool could_improve(float q1, float q0, float dd) const {
+        const float m = fmaxf(fminf(fmaf(-0x1p-18f, q1 + dd, q0), q1), 0.f);
+        const float lb = sqrtf(m) * kSureDown - sqrtf(dd) * kSureUp;
+        return !(fminf(dd, q1) > kSureMin && lb > 0.f && lb * lb * kSureDown > q);
+    }
+};
+
+__device__ __forceinline__ double unit64(const OrbitScale &s) { return __hiloint2double((1023 - 55 + s.e) << 20, 0); }
+__device__ __forceinline__ bool in_range32(float ra, float rb, float rmax) {
+    return fmaxf(ra, rb) < rmax && fminf(ra, rb) > kOrbit32MinR2;
+}
+
+// the scale of a clone's two orbits (false: none, NaN and infinities included)
+__device__ __forceinline__ bool clone_scale(const double *p, int steps, double dt, OrbitScale &s) {
+    double reach = 0.0, sum = 0.0;
+#pragma unroll
+    for (int o = 0; o < 12; o += 6) {
+        const double x = fmax(fabs(p[o]), fmax(fabs(p[o + 1]), fabs(p[o + 2])));
+        const double v = fmax(fabs(p[o + 3]), fmax(fabs(p[o + 4]), fabs(p[o + 5]))) * fabs(dt);
+        reach = fmax(reach, fmax(2.0 * x + 2.0 * v * steps + 20.0, 256.0 * v));
+    }
+#pragma unroll
+    for (int j = 0; j < 12; j++) sum += p[j];                 // fmax passes over NaN
+    return fabs(sum) < 1e300 && orbit32_scale(reach, dt, s);
+}
+
 struct Clone32 {
     Orbit32 a, b;
     Force32 K;
     OrbitScale s;
-    Approach r;
-    float q, rmax;           // r.best^2 in squared high-word units; r2 limit
-    int tie;                 // > 0: the record is a tie that the FP64 trace of this many steps decides
-    bool pend, ok;
-    __device__ __forceinline__ double unit() const { return __hiloint2double((1023 - 55 + s.e) << 20, 0); }
-    __device__ __forceinline__ void set_q() {
-        const float f = (float)(r.best * __hiloint2double((1023 + 23 - s.e) << 20, 0));
-        q = f * f;
-    }
+    Near32 n;
+    float rmax;              // r2 limit
+    bool ok;
     // false: not an orbit for these units (traced in FP64)
     __device__ __forceinline__ bool start(const double *__restrict__ ps, int steps, double dt) {
         double p[12];
 #pragma unroll
         for (int j = 0; j < 12; j++) p[j] = ps[j];
-        double reach = 0.0;
-#pragma unroll
-        for (int o = 0; o < 12; o += 6) {
-            const double x = fmax(fabs(p[o]), fmax(fabs(p[o + 1]), fabs(p[o + 2])));
-            const double v = fmax(fabs(p[o + 3]), fmax(fabs(p[o + 4]), fabs(p[o + 5]))) * fabs(dt);
-            reach = fmax(reach, fmax(2.0 * x + 2.0 * v * steps + 20.0, 256.0 * v));
-        }
-        double sum = 0.0;                                     // NaN and infinities, which fmax passes over
-#pragma unroll
-        for (int j = 0; j < 12; j++) sum += p[j];
-        if (!(fabs(sum) < 1e300)) reach = sum * 0.0 + 1e300;
-        pend = false;
-        tie = 0;
-        ok = orbit32_scale(reach, dt, s);
+        n.pend = false;
+        n.tie = 0;
+        ok = clone_scale(p, steps, dt, s);
         if (!ok) return false;
         K = force32_constants<MwModel32>(dt, s);
         rmax = orbit32_max_r2(s);
         float ra, rb;
         orbit32_start<MwModel32>(a, K, HaloTable32(), s, p, p + 3, dt, ra);
         orbit32_start<MwModel32>(b, K, HaloTable32(), s, p + 6, p + 9, dt, rb);
-        in_range(ra, rb);
-        const double rx = p[0] - p[6], ry = p[1] - p[7], rz = p[2] - p[8];
-        r.best = sqrt(fma(rx, rx, fma(ry, ry, rz * rz)));
-        r.tbest = 0.0;
-        const double ux = p[3] - p[9], uy = p[4] - p[10], uz = p[5] - p[11];
-        r.vbest = sqrt(fma(ux, ux, fma(uy, uy, uz * uz)));
-        set_q();
+        ok = in_range32(ra, rb, rmax);
+        n.start(p, s);
         return true;
-    }
-    __device__ __forceinline__ void in_range(float ra, float rb) {
-        ok = ok && fmaxf(ra, rb) < rmax && fminf(ra, rb) > kOrbit32MinR2;
     }
     __device__ __forceinline__ void step(int i, double dt) {
         const I3 sa = {a.wx >> 6, a.wy >> 6, a.wz >> 6}, sb = {b.wx >> 6, b.wy >> 6, b.wz >> 6};
@@ -476,57 +488,163 @@ struct Clone32 {
         const HaloTable32 T;
         const Acc64i A = accel32<MwModel32>(K, T, s.c, a.x, a.y, a.z, ra);
         const Acc64i B = accel32<MwModel32>(K, T, s.c, b.x, b.y, b.z, rb);
-        in_range(ra, rb);
+        ok = ok && in_range32(ra, rb, rmax);
         const I3 d = sa - sb, r1 = {a.x - b.x, a.y - b.y, a.z - b.z};
         const float dx = fixed_to_f32(d.x), dy = fixed_to_f32(d.y), dz = fixed_to_f32(d.z);
         const float rx = fixed_to_f32(r1.x), ry = fixed_to_f32(r1.y), rz = fixed_to_f32(r1.z);
-        const float dd = fmaf(dx, dx, fmaf(dy, dy, dz * dz)), q1 = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
-        const float b1 = fmaf(rx, dx, fmaf(ry, dy, rz * dz)), a0 = b1 - dd;
-        const float t = fminf(dd, q1) > kSureMin ? kSure2 * dd * (q1 + dd) : __int_as_float(0x7f800000);
-        if (a0 > 0.f && a0 * a0 > t) {
-            if (pend) approach_ended(sa, sb, i, dt);
-        } else {
-            const bool in = b1 < 0.f && b1 * b1 > t;
-            if (in && (pend || q1 * kSureUp < q)) {
-                pend = true;
-                tie = 0;
-                q = q1;
-            } else if (in ? q1 * kSureDown <= q : (pend || could_improve(q1, fmaf(-2.f, b1, q1 + dd), dd))) {
-                const I3 v2 = {2 * (a.wx - b.wx) + (A.x - B.x), 2 * (a.wy - b.wy) + (A.y - B.y),
-                               2 * (a.wz - b.wz) + (A.z - B.z)};
-                const int got = segment64(r1, d, v2, i, dt, unit(), pend, r, &tie);
-                if (got == kSegAtR0) approach_ended(sa, sb, i, dt);
-                pend = false;
-                set_q();
-            }
-        }
+        if (ok)
+            n.step(fmaf(dx, dx, fmaf(dy, dy, dz * dz)), fmaf(rx, rx, fmaf(ry, ry, rz * rz)),
+                   fmaf(rx, dx, fmaf(ry, dy, rz * dz)), s,
+                   [&](bool at_r0, Approach &r, int *tie) {
+                       const I3 v2 = {2 * (a.wx - b.wx) + (A.x - B.x), 2 * (a.wy - b.wy) + (A.y - B.y),
+                                      2 * (a.wz - b.wz) + (A.z - B.z)};
+                       return segment64(r1, d, v2, i, dt, unit64(s), at_r0, r, tie);
+                   },
+                   [&]() {
+                       Orbit32 a0 = a, b0 = b;
+                       a0.x -= sa.x; a0.y -= sa.y; a0.z -= sa.z;
+                       b0.x -= sb.x; b0.y -= sb.y; b0.z -= sb.z;
+                       return vertex64(a0, b0, K, s, i - 1, dt);
+                   });
         a.wx += A.x; a.wy += A.y; a.wz += A.z;
         b.wx += B.x; b.wy += B.y; b.wz += B.z;
     }
-    // the pending record at the start of step i (the orbits have moved on by sa, sb)
-    __device__ __forceinline__ void approach_ended(const I3 &sa, const I3 &sb, int i, double dt) {
-        Orbit32 a0 = a, b0 = b;
-        a0.x -= sa.x; a0.y -= sa.y; a0.z -= sa.z;
-        b0.x -= sb.x; b0.y -= sb.y; b0.z -= sb.z;
-        r = vertex64(a0, b0, K, s, i - 1, dt);
-        pend = false;
-        set_q();
-    }
-    // whether a segment between squared distances q0 and q1 can come nearer than the best: no point of it is nearer
-    // than the nearer end less its length
-    __device__ __forceinline__ bool could_improve(float q1, float q0, float dd) const {
-        const float m = fmaxf(fminf(fmaf(-0x1p-18f, q1 + dd, q0), q1), 0.f);
-        const float lb = sqrtf(m) * kSureDown - sqrtf(dd) * kSureUp;
-        return !(fminf(dd, q1) > kSureMin && lb > 0.f && lb * lb * kSureDown > q);
-    }
     // after the last step: the approach may still be on
     __device__ __forceinline__ void finish(int steps, double dt) {
-        if (pend) r = vertex64(a, b, K, s, steps, dt);
-        tie = min(tie, steps);
+        if (n.pend) n.r = vertex64(a, b, K, s, steps, dt);
     }
     // the steps the FP64 trace takes for this clone's record (0: none, the record stands)
-    __device__ __forceinline__ int fp64_steps(int steps) const { return ok ? tie : max(steps, 1); }
+    __device__ __forceinline__ int fp64_steps(int steps) const { return ok ? min(n.tie, steps) : max(steps, 1); }
 };
+
+// The same clone on eight lanes (quad_accel32: target on lanes 0-3 of the eight, cluster on 4-7): the same bits.
+struct QuadClone32 {
+    long long x, w;          // the lane's coordinate and displacement
+    F3 k;
+    OrbitScale s;
+    Near32 n;                // alike on the eight lanes
+    float rmax;
+    bool ok;
+    __device__ __forceinline__ static unsigned group() { return 0xffu << (threadIdx.x & 24u); }
+    // lanes 0, 1, 2 of the eight hold the target's v, lanes 4, 5, 6 the cluster's: the differences, on every lane
+    __device__ __forceinline__ static I3 diff3(long long v) {
+        const unsigned m = group();
+        const long long d = v - __shfl_xor_sync(m, v, 4);
+        return I3{__shfl_sync(m, d, 0, 8), __shfl_sync(m, d, 1, 8), __shfl_sync(m, d, 2, 8)};
+    }
+    __device__ __forceinline__ static Orbit32 gather(long long x, long long w, int o) {
+        const unsigned m = group();
+        return Orbit32{__shfl_sync(m, x, o, 8), __shfl_sync(m, x, o + 1, 8), __shfl_sync(m, x, o + 2, 8),
+                       __shfl_sync(m, w, o, 8), __shfl_sync(m, w, o + 1, 8), __shfl_sync(m, w, o + 2, 8)};
+    }
+    __device__ __forceinline__ Approach vertex(long long x0, int i, double dt) const {
+        const Orbit32 a = gather(x0, w, 0), b = gather(x0, w, 4);
+        return vertex64(a, b, force32_constants<MwModel32>(dt, s), s, i, dt);
+    }
+    __device__ __forceinline__ void start(const double *__restrict__ ps, int steps, double dt, int role) {
+        double p[12];
+#pragma unroll
+        for (int j = 0; j < 12; j++) p[j] = ps[j];
+        ok = clone_scale(p, steps, dt, s);
+        if (!ok) s = OrbitScale{0x1p-23f, 0};                 // (traced along with its warp, and again in FP64)
+        k = quad_constant(force32_constants<MwModel32>(ok ? dt : 0.05, s), role);
+        rmax = orbit32_max_r2(s);
+        const int o = threadIdx.x & 4 ? 6 : 0;
+        const double q = role == 0 ? ps[o] : (role == 1 ? ps[o + 1] : ps[o + 2]);
+        const double v = role == 0 ? ps[o + 3] : (role == 1 ? ps[o + 4] : ps[o + 5]);
+        x = ok && role < 3 ? f64_to_i64(q * ldexp(1.0, 55 - s.e)) : 0;
+        float r2;
+        const long long a = quad_accel32(k, s.c, x, role, r2);
+        w = (ok && role < 3 ? displacement(v, dt, ldexp(1.0, 61 - s.e)) + a / 2 : 0) + 32;
+        const float rb = __shfl_xor_sync(0xffffffffu, r2, 4);        // (every lane, whatever its ok)
+        ok = ok && in_range32(r2, rb, rmax);
+        n.start(p, s);
+    }
+    __device__ __forceinline__ void step(int i, double dt, int role) {
+        const unsigned all = 0xffffffffu;
+        const long long sw = w >> 6;
+        x += sw;
+        float r2;
+        const long long a = quad_accel32(k, s.c, x, role, r2);
+        const float rb = __shfl_xor_sync(all, r2, 4);                 // (every lane, whatever its ok)
+        ok = ok && in_range32(r2, rb, rmax);
+        const float fd = fixed_to_f32(sw - __shfl_xor_sync(all, sw, 4)), fr = fixed_to_f32(x - __shfl_xor_sync(all, x, 4));
+        const float dx = __shfl_sync(all, fd, 0, 8), dy = __shfl_sync(all, fd, 1, 8), dz = __shfl_sync(all, fd, 2, 8);
+        const float rx = __shfl_sync(all, fr, 0, 8), ry = __shfl_sync(all, fr, 1, 8), rz = __shfl_sync(all, fr, 2, 8);
+        if (ok)
+            n.step(fmaf(dx, dx, fmaf(dy, dy, dz * dz)), fmaf(rx, rx, fmaf(ry, ry, rz * rz)),
+                   fmaf(rx, dx, fmaf(ry, dy, rz * dz)), s,
+                   [&](bool at_r0, Approach &r, int *tie) {
+                       return segment64(diff3(x), diff3(sw), diff3(2 * w + a), i, dt, unit64(s), at_r0, r, tie);
+                   },
+                   [&]() { return vertex(x - sw, i - 1, dt); });
+        w += a;
+    }
+    __device__ __forceinline__ void finish(int steps, double dt) {
+        if (n.pend) n.r = vertex(x, steps, dt);
+    }
+    __device__ __forceinline__ int fp64_steps(int steps) const { return ok ? min(n.tie, steps) : max(steps, 1); }
+};
+
+// Coarse tracks of the prefilter (reference track, src/phygas.c:98-111): the nominal orbit of each object from ps
+// (6 doubles per object); pos[k][3][N] = the position after 10 k KDK steps of -0.05 Myr, for k < npts[i].  On the FP32
+// and integer units, four lanes per orbit (quad_accel32), one warp per block: a few to a few thousand orbits, whose steps'
+// latency is the time.  Orbits outside the units' range are traced again in FP64 (quad_accel).  The tracks of 3 pulsars and
+// their pair tests: 4.7 -> 0.8 ms.
+static __global__ void __launch_bounds__(32) k_coarse_tracks(int N, const double *__restrict__ ps,
+                                                             const int *__restrict__ npts, double *__restrict__ pos) {
+    const unsigned all = 0xffffffffu;
+    const size_t NN = N;
+    const int t = blockIdx.x * 8 + (threadIdx.x >> 2), role = threadIdx.x & 3, c = role < 3 ? role : 2;
+    const int i = min(t, N - 1);                              // lanes past the end repeat the last orbit
+    const bool mine = t < N && role < 3;
+    const double *q = ps + 6 * (size_t)i;
+    const int n = npts[i], nw = __reduce_max_sync(all, n);
+    constexpr double dt = -kStepMyr / kSub, h = 0.5 * dt;
+    double p12[12];
+#pragma unroll
+    for (int j = 0; j < 6; j++) p12[j] = p12[6 + j] = q[j];
+    OrbitScale s;
+    bool ok = clone_scale(p12, (n - 1) * kSub, dt, s);
+    if (!ok) s = OrbitScale{0x1p-23f, 0};
+    const F3 k = quad_constant(force32_constants<MwModel32>(dt, s), role);
+    const float rmax = orbit32_max_r2(s);
+    const double unit = unit64(s);
+    long long x = ok && role < 3 ? f64_to_i64(q[c] * ldexp(1.0, 55 - s.e)) : 0;
+    float r2;
+    const long long a0 = quad_accel32(k, s.c, x, role, r2);
+    ok = ok && in_range32(r2, r2, rmax);
+    long long w = (ok && role < 3 ? displacement(q[3 + c], dt, ldexp(1.0, 61 - s.e)) + a0 / 2 : 0) + 32;
+    for (int j = 0; j < nw; j++) {
+        if (j > 0) {
+#pragma unroll 1
+            for (int m = 0; m < kSub; m++) {
+                x += w >> 6;
+                w += quad_accel32(k, s.c, x, role, r2);
+                ok = ok && (j >= n || in_range32(r2, r2, rmax));
+            }
+        }
+        if (mine && j < n) pos[((size_t)j * 3 + c) * NN + i] = j ? (double)x * unit : q[c];
+    }
+    if (!__any_sync(all, !ok)) return;
+    QuadOrbit o;
+    o.q = role < 3 ? q[c] : 0.0;
+    o.v = role < 3 ? q[3 + c] : 0.0;
+    o.init(role);
+    for (int j = 0; j < nw; j++) {
+        if (j > 0) {
+#pragma unroll 1
+            for (int m = 0; m < kSub; m++) o.kdk(dt, h, role);
+        }
+        if (mine && !ok && j < n) pos[((size_t)j * 3 + c) * NN + i] = o.q;
+    }
+}
+
+cudaError_t launch_coarse_tracks(cudaStream_t st, int N, const double *ps, const int *npts, double *pos) {
+    if (N <= 0) return cudaSuccess;
+    k_coarse_tracks<<<(N + 7) / 8, 32, 0, st>>>(N, ps, npts, pos);
+    return cudaGetLastError();
+}
 
 // The clones of a warp that take the FP64 trace: n steps of each lane's clone (0: none; every lane calls).  A few are
 // traced by the whole warp one after the other, more (a step length or a reach outside the FP32 orbit's) lane by lane:
@@ -550,16 +668,16 @@ __device__ __forceinline__ void trace_fp64(const double *ps, int n, int steps, d
 // a lane's clone (every lane of the warp calls; active: it has one)
 __device__ __forceinline__ Approach trace_clone(bool active, const double *__restrict__ ps, int steps, double dt) {
     Clone32 c;
-    c.ok = c.pend = false;
-    c.tie = 0;
+    c.ok = c.n.pend = false;
+    c.n.tie = 0;
     if (active && c.start(ps, steps, dt)) {
 #pragma unroll 1
         for (int i = 1; i <= steps; i++) c.step(i, dt);
     }
     if (active && c.ok) c.finish(steps, dt);
     __syncwarp();
-    trace_fp64(ps, active ? c.fp64_steps(steps) : 0, steps, dt, c.r);
-    return c.r;
+    trace_fp64(ps, active ? c.fp64_steps(steps) : 0, steps, dt, c.n.r);
+    return c.n.r;
 }
 
 // ---- reduction of one pair (m clones) ---------------------------------------------------------------------------
@@ -674,40 +792,14 @@ __device__ void reduce_dispatch(const McPairs &P, int p, double *smem_w, int lan
     else warp_reduce_pair<32>(b, t, v, m, r50, rt, smem_w, out, lane);
 }
 
-// Persistent clone kernel.  items[q] = (pair, first clone, count <= 32), longest trace first.  No warp ever waits
-// for another: a warp takes the next item with one atomic, and the warp whose item completes a pair's count (an
-// atomic per item, after a fence) reduces that pair.
-__global__ void __launch_bounds__(kMcThreads) k_pair_mc(McPairs P) {
-    __shared__ double smem[kMcThreads / 32][1024];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (;;) {
-        int q = 0;
-        if (lane == 0) q = atomicAdd(P.qhead, 1);
-        q = __shfl_sync(0xffffffffu, q, 0);
-        if (q >= P.n_items) break;
-        const int4 it = P.items[q];   // x = pair, y = first clone, z = count
-        const int p = it.x;
-        const int c = it.y + lane;
-        const Approach r = trace_clone(lane < it.z, P.ps + (size_t)c * 12, P.steps[p], P.dt[p]);
-        if (lane < it.z) {
-            P.cres[c] = r.best;
-            P.cres[P.n_clones + c] = r.tbest;
-            P.cres[2 * (size_t)P.n_clones + c] = r.vbest;
-        }
-        __threadfence();
-        __syncwarp();
-        int last = 0;
-        if (lane == 0) {
-            const int m = P.clone_off[p + 1] - P.clone_off[p];
-            last = atomicAdd(P.done + p, it.z) + it.z == m;
-        }
-        last = __shfl_sync(0xffffffffu, last, 0);
-        if (last) {
-            __threadfence();
-            const int m = P.clone_off[p + 1] - P.clone_off[p];
-            if (m <= 1024) reduce_dispatch(P, p, smem[w], lane);
-        }
-    }
+// A warp's first item goes by its place in the grid, the next ones by the queue (k_mc_prep sets its head past the first
+// ones).  With all of them from the queue, the SMs whose warps came first took a small batch's items for themselves, 16
+// warps where others had none: 1 pair x 20,000 clones took 3.4 to 4.4 ms, spread out 2.2 ms.
+__device__ __forceinline__ int first_item() { return blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); }
+__device__ __forceinline__ int next_item(const McPairs &P) {
+    int q = 0;
+    if ((threadIdx.x & 31) == 0) q = atomicAdd(P.qhead, 1);
+    return __shfl_sync(0xffffffffu, q, 0);
 }
 
 // Persistent clone tracing for batches replayed from a captured graph: parameters read from device memory, and the
@@ -720,11 +812,7 @@ template <int WARPS, int CPL, int MINB>
 __global__ void __launch_bounds__(WARPS * 32, MINB > 1 ? MINB : 16 / (WARPS * CPL)) k_pair_mc_t(const McPairs *__restrict__ Pd) {
     const McPairs P = *Pd;
     const int lane = threadIdx.x & 31;
-    for (;;) {
-        int q = 0;
-        if (lane == 0) q = atomicAdd(P.qhead, 1);
-        q = __shfl_sync(0xffffffffu, q, 0);
-        if (q >= P.n_items) break;
+    for (int q = first_item(); q < P.n_items; q = next_item(P)) {
         const int4 it = P.items[q];   // x = pair, y = first clone, z = count
         const int p = it.x;
         const int steps = P.steps[p];
@@ -749,20 +837,46 @@ __global__ void __launch_bounds__(WARPS * 32, MINB > 1 ? MINB : 16 / (WARPS * CP
             const int cc = it.y + (mine ? lane + 32 * j : 0);
             if (c[j].ok) c[j].finish(steps, dt);
             __syncwarp();
-            trace_fp64(P.ps + (size_t)cc * 12, mine ? c[j].fp64_steps(steps) : 0, steps, dt, c[j].r);
+            trace_fp64(P.ps + (size_t)cc * 12, mine ? c[j].fp64_steps(steps) : 0, steps, dt, c[j].n.r);
             if (!mine) continue;
-            P.cres[cc] = c[j].r.best;
-            P.cres[P.n_clones + cc] = c[j].r.tbest;
-            P.cres[2 * (size_t)P.n_clones + cc] = c[j].r.vbest;
+            P.cres[cc] = c[j].n.r.best;
+            P.cres[P.n_clones + cc] = c[j].n.r.tbest;
+            P.cres[2 * (size_t)P.n_clones + cc] = c[j].n.r.vbest;
         }
     }
 }
 
-// before k_pair_mc_t: queue head zeroed, empty results for pairs without clones
-__global__ void k_mc_prep(const McPairs *__restrict__ Pd) {
+// The same with eight lanes per clone, items of up to four clones: for batches of few clones, where a step's latency
+// counts (kMcQuadClones).
+__global__ void __launch_bounds__(kMcQuadWarps * 32) k_pair_mc_quad(const McPairs *__restrict__ Pd) {
+    const McPairs P = *Pd;
+    const int lane = threadIdx.x & 31, role = threadIdx.x & 3, e = lane >> 3;
+    for (int q = first_item(); q < P.n_items; q = next_item(P)) {
+        const int4 it = P.items[q];   // x = pair, y = first clone, z = count
+        const int p = it.x, steps = P.steps[p], cc = it.y + min(e, it.z - 1);
+        const double dt = P.dt[p];
+        QuadClone32 c;
+        c.start(P.ps + (size_t)cc * 12, steps, dt, role);
+        if (__any_sync(0xffffffffu, c.ok)) {
+#pragma unroll 1
+            for (int i = 1; i <= steps; i++) c.step(i, dt, role);
+        }
+        if (c.ok) c.finish(steps, dt);
+        __syncwarp();
+        const bool mine = (lane & 7) == 0 && e < it.z;
+        trace_fp64(P.ps + (size_t)cc * 12, mine ? c.fp64_steps(steps) : 0, steps, dt, c.n.r);
+        if (!mine) continue;
+        P.cres[cc] = c.n.r.best;
+        P.cres[P.n_clones + cc] = c.n.r.tbest;
+        P.cres[2 * (size_t)P.n_clones + cc] = c.n.r.vbest;
+    }
+}
+
+// before k_pair_mc_t: queue head past the first items of its warps, empty results for pairs without clones
+__global__ void k_mc_prep(const McPairs *__restrict__ Pd, int warps) {
     const McPairs P = *Pd;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t == 0) *P.qhead = 0;
+    if (t == 0) *P.qhead = warps;
     for (int p = t; p < P.n_pairs; p += gridDim.x * blockDim.x) {
         if (P.clone_off[p + 1] - P.clone_off[p] > 0) continue;
         PhResultDev o;
@@ -789,14 +903,17 @@ struct McVariant {
     int warps, cpl, min_blocks;
     void (*fn)(const McPairs *);
 };
+// the last entry: eight lanes per clone (not one of the tuner's shapes)
 const McVariant kMcVariants[] = {
     {4, 1, 1, k_pair_mc_t<4, 1, 1>}, {2, 1, 1, k_pair_mc_t<2, 1, 1>}, {8, 1, 1, k_pair_mc_t<8, 1, 1>},
     {4, 2, 1, k_pair_mc_t<4, 2, 1>}, {2, 2, 1, k_pair_mc_t<2, 2, 1>}, {8, 2, 1, k_pair_mc_t<8, 2, 1>},
     {4, 1, 5, k_pair_mc_t<4, 1, 5>}, {4, 1, 6, k_pair_mc_t<4, 1, 6>}, {8, 1, 3, k_pair_mc_t<8, 1, 3>},
+    {kMcQuadWarps, 0, 1, k_pair_mc_quad},
 };
 }  // namespace
 
-int mc_variants() { return (int)(sizeof kMcVariants / sizeof kMcVariants[0]); }
+int mc_variants() { return (int)(sizeof kMcVariants / sizeof kMcVariants[0]) - 1; }
+int mc_quad_variant() { return mc_variants(); }
 
 void mc_variant_shape(int v, int &warps, int &cpl, int &min_blocks) {
     warps = kMcVariants[v].warps;
@@ -815,7 +932,7 @@ cudaError_t mc_variant_grid(int v, int sms, int &grid) {
 
 // prep, trace (variant v on a persistent grid) and reduce on one stream; reduce_grid blocks of kMcThreads
 cudaError_t launch_mc(int v, int grid, int prep_grid, int reduce_grid, cudaStream_t st, const McPairs *Pd) {
-    k_mc_prep<<<prep_grid, 256, 0, st>>>(Pd);
+    k_mc_prep<<<prep_grid, 256, 0, st>>>(Pd, grid * kMcVariants[v].warps);
     kMcVariants[v].fn<<<grid, kMcVariants[v].warps * 32, 0, st>>>(Pd);
     k_pair_reduce_dev<<<reduce_grid, kMcThreads, 0, st>>>(Pd);
     return cudaGetLastError();
@@ -840,137 +957,173 @@ __device__ __forceinline__ unsigned long long reduce_key(const double *src, int 
     return (unsigned long long)__double_as_longlong(v);
 }
 
-// The k-th smallest (0-based) of a pair's m values of array `which`, read from global memory by the whole block: an
-// MSB radix selection, 8 bits a pass, each pass counting the values that share the prefix found so far.  Exact: the
-// element a sort would put at index k.  For pairs too large to sort in shared memory.
-__device__ double radix_select(const double *src, int which, int m, int k) {
-    __shared__ unsigned hist[256];
-    __shared__ unsigned long long s_prefix;
-    __shared__ int s_k;
-    if (threadIdx.x == 0) { s_prefix = 0; s_k = k; }
-    unsigned long long mask = 0;
-    for (int shift = 56; shift >= 0; shift -= 8) {
-        for (int b = threadIdx.x; b < 256; b += blockDim.x) hist[b] = 0;
+// Order statistics of a pair's m values of array `which`, read from global memory by the whole block: an MSB radix
+// selection of all kRanks ranks (rank[r], 0-based) at once, 8 bits a pass, starting below the bits that all values share.
+// A pass counts the values under each prefix that some rank still follows; a warp per rank then finds its digit.  Exact:
+// the elements that a sort would put there.  For pairs too large to sort in shared memory: 20,000 values in about 9
+// passes, where a selection per rank and array in turn, a digit found by one thread, read them 144 times (1.86 ms).
+constexpr int kRanks = 6, kReduceThreads = 1024;
+__device__ void radix_select(const double *src, int which, int m, const int *rank, double *value) {
+    __shared__ unsigned hist[kRanks][256];
+    __shared__ unsigned long long s_prefix[kRanks], s_min, s_max;
+    __shared__ int s_left[kRanks], s_group[kRanks];             // rank within its prefix; the first rank of its prefix
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    if (tid == 0) { s_min = ~0ull; s_max = 0; }
+    __syncthreads();
+    unsigned long long lo = ~0ull, hi = 0;
+    for (int e = tid; e < m; e += blockDim.x) {
+        const unsigned long long key = reduce_key(src, which, e);
+        lo = kmin(lo, key);
+        hi = kmax(hi, key);
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        lo = kmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+        hi = kmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    }
+    if (lane == 0) { atomicMin(&s_min, lo); atomicMax(&s_max, hi); }
+    __syncthreads();
+    const int top = s_min == s_max ? 0 : 64 - __clzll((long long)(s_min ^ s_max));      // bits that differ
+    unsigned long long mask = top == 64 ? 0ull : ~0ull << top;
+    if (tid < kRanks) { s_prefix[tid] = s_min & mask; s_left[tid] = rank[tid]; }
+    __syncthreads();
+    for (int shift = top - 8; mask != ~0ull; shift -= 8) {
+        const int sh = shift > 0 ? shift : 0;                    // the last pass takes the bits that are left
+        const unsigned long long digits = ~mask & (~0ull << sh);
+        if (tid < kRanks) {
+            int g = 0;
+            while (s_prefix[g] != s_prefix[tid]) g++;
+            s_group[tid] = g;
+        }
+        for (int b = tid; b < kRanks * 256; b += blockDim.x) (&hist[0][0])[b] = 0;
         __syncthreads();
-        const unsigned long long prefix = s_prefix;
-        for (int e = threadIdx.x; e < m; e += blockDim.x) {
-            const unsigned long long key = reduce_key(src, which, e);
-            if ((key & mask) == prefix) atomicAdd(&hist[(key >> shift) & 255u], 1u);
+        for (int e = tid; e < m; e += blockDim.x) {
+            const unsigned long long key = reduce_key(src, which, e), pre = key & mask;
+            const unsigned d = (unsigned)((key & digits) >> sh);
+#pragma unroll
+            for (int g = 0; g < kRanks; g++)
+                if (s_group[g] == g && pre == s_prefix[g]) atomicAdd(&hist[g][d], 1u);
         }
         __syncthreads();
-        if (threadIdx.x == 0) {
-            int kk = s_k, b = 0;
-            for (; b < 255 && kk >= (int)hist[b]; b++) kk -= (int)hist[b];
-            s_k = kk;
-            s_prefix = prefix | ((unsigned long long)b << shift);
+        if (w < kRanks) {                                        // warp w: rank w's digit, 8 bins a lane
+            const unsigned *h = hist[s_group[w]] + 8 * lane;
+            int c[8], sum = 0;
+#pragma unroll
+            for (int b = 0; b < 8; b++) { c[b] = (int)h[b]; sum += c[b]; }
+            int before = sum;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int t = __shfl_up_sync(0xffffffffu, before, o);
+                if (lane >= o) before += t;
+            }
+            before -= sum;
+            const int k = s_left[w];
+            const unsigned long long prefix = s_prefix[w];
+            __syncwarp();
+            if (k >= before && k < before + sum) {
+                int b = 0;
+                for (int left = k - before; left >= c[b]; b++) left -= c[b];
+                for (int q = 0; q < b; q++) before += c[q];
+                s_left[w] = k - before;
+                s_prefix[w] = prefix | (unsigned long long)(8 * lane + b) << sh;
+            }
         }
-        mask |= 255ull << shift;
+        mask |= digits;
         __syncthreads();
     }
-    const double v = __longlong_as_double((long long)s_prefix);
+    if (tid < kRanks) value[tid] = __longlong_as_double((long long)s_prefix[tid]);
     __syncthreads();
-    return v;
 }
 
-// interp_q of the sorted values, the two order statistics it reads found by radix_select
-__device__ double select_q(const double *src, int which, int m, double q) {
-    const double pos = __dmul_rn(q, (double)(m - 1));
-    const int i = (int)pos;
-    if (i >= m - 1) return radix_select(src, which, m, m - 1);
-    const double a = radix_select(src, which, m, i), b = radix_select(src, which, m, i + 1);
-    return __dadd_rn(a, __dmul_rn(__dsub_rn(pos, (double)i), __dsub_rn(b, a)));
-}
-
-// pairs of 0 clones never get an item: their (empty) result is written here, with the big-pair reduction.  Pairs of
-// up to kSortMax clones are sorted in shared memory (launched with room for the batch's largest such pair); larger
-// pairs take their order statistics by radix selection from global memory.
-__global__ void k_pair_reduce_big(McPairs P) {
+// Pairs of more than 1024 clones (and the empty result of pairs without clones), a block per pair and array: sorted in
+// shared memory up to kSortMax clones (launched with room for the batch's largest such pair), beyond that by radix
+// selection from global memory.
+__global__ void __launch_bounds__(kReduceThreads) k_pair_reduce_big(McPairs P) {
     extern __shared__ double sm[];
-    const int p = blockIdx.x;
+    const int p = blockIdx.x / 3, which = blockIdx.x % 3;
     const int m = P.clone_off[p + 1] - P.clone_off[p];
     if (m > 0 && m <= 1024) return;
     PhResultDev *out = P.res + p;
+    double *quant = which == 0 ? &out->d05 : (which == 1 ? &out->t05 : &out->v05);
     if (m <= 0) {
         if (threadIdx.x == 0) {
-            PhResultDev o;
-            o.n = 0;
-            o.pad = 0;
-            o.d05 = o.d50 = o.d95 = o.t05 = o.t50 = o.t95 = o.v05 = o.v50 = o.v95 = o.f_r50 = o.f_rtot = 0.0;
-            *out = o;
+            quant[0] = quant[1] = quant[2] = 0.0;
+            if (which == 0) { out->n = 0; out->pad = 0; out->f_r50 = out->f_rtot = 0.0; }
+        }
+        return;
+    }
+    const size_t o = P.clone_off[p];
+    const double *src = P.cres + (size_t)which * P.n_clones + o;
+    if (which == 0) {
+        __shared__ int c50, ctot;
+        if (threadIdx.x == 0) { c50 = 0; ctot = 0; }
+        __syncthreads();
+        const double r50 = P.r50_pc[p], rtot = P.rtot_pc[p];
+        int l50 = 0, ltot = 0;
+        for (int e = threadIdx.x; e < m; e += blockDim.x) {
+            const double v = __dmul_rn(src[e], 1000.0);
+            l50 += v < r50;
+            ltot += v < rtot;
+        }
+        l50 = __reduce_add_sync(0xffffffffu, l50);
+        ltot = __reduce_add_sync(0xffffffffu, ltot);
+        if ((threadIdx.x & 31) == 0) { atomicAdd(&c50, l50); atomicAdd(&ctot, ltot); }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            out->n = m;
+            out->pad = 0;
+            out->f_r50 = __ddiv_rn((double)c50, (double)m);
+            out->f_rtot = __ddiv_rn((double)ctot, (double)m);
+        }
+    }
+    if (m > kSortMax) {
+        __shared__ int rank[kRanks];
+        __shared__ double value[kRanks];
+        if (threadIdx.x < 3) {
+            const double pos = __dmul_rn(threadIdx.x == 0 ? 0.05 : (threadIdx.x == 1 ? 0.5 : 0.95), (double)(m - 1));
+            const int i = min((int)pos, m - 1);
+            rank[2 * threadIdx.x] = i;
+            rank[2 * threadIdx.x + 1] = min(i + 1, m - 1);
+        }
+        __syncthreads();
+        radix_select(src, which, m, rank, value);
+        if (threadIdx.x < 3) {
+            const double pos = __dmul_rn(threadIdx.x == 0 ? 0.05 : (threadIdx.x == 1 ? 0.5 : 0.95), (double)(m - 1));
+            const int i = (int)pos;
+            const double a = value[2 * threadIdx.x], b = value[2 * threadIdx.x + 1];
+            quant[threadIdx.x] = i >= m - 1 ? a : __dadd_rn(a, __dmul_rn(__dsub_rn(pos, (double)i), __dsub_rn(b, a)));
         }
         return;
     }
     int n2 = 1;
     while (n2 < m) n2 <<= 1;
     unsigned long long *key = reinterpret_cast<unsigned long long *>(sm);
-    const size_t o = P.clone_off[p];
-    __shared__ int c50, ctot;
-    __shared__ double res[9];
-    if (threadIdx.x == 0) { c50 = 0; ctot = 0; }
+    for (int e = threadIdx.x; e < n2; e += blockDim.x) key[e] = e < m ? reduce_key(src, which, e) : 0x7ff0000000000000ULL;
     __syncthreads();
-    if (m > kSortMax) {
-        int l50 = 0, ltot = 0;
-        for (int e = threadIdx.x; e < m; e += blockDim.x) {
-            const double v = __dmul_rn(P.cres[o + e], 1000.0);
-            l50 += v < P.r50_pc[p];
-            ltot += v < P.rtot_pc[p];
-        }
-        atomicAdd(&c50, l50);
-        atomicAdd(&ctot, ltot);
-        for (int which = 0; which < 3; which++) {
-            const double *src = P.cres + (size_t)which * P.n_clones + o;
-            const double q05 = select_q(src, which, m, 0.05), q50 = select_q(src, which, m, 0.5),
-                         q95 = select_q(src, which, m, 0.95);
-            if (threadIdx.x == 0) { res[3 * which] = q05; res[3 * which + 1] = q50; res[3 * which + 2] = q95; }
-        }
-        __syncthreads();
-        n2 = 0;                             // nothing left to sort below
-    }
-    for (int which = 0; which < 3 && n2 > 0; which++) {
-        const double *src = P.cres + (size_t)which * P.n_clones + o;
-        int l50 = 0, ltot = 0;
-        for (int e = threadIdx.x; e < n2; e += blockDim.x) {
-            double v = 0.0;
-            if (e < m) {
-                v = src[e];
-                if (which == 0) { v = __dmul_rn(v, 1000.0); l50 += v < P.r50_pc[p]; ltot += v < P.rtot_pc[p]; }
-                else if (which == 2) v = __dmul_rn(v, kKms);
+    for (int k = 2; k <= n2; k <<= 1)
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            for (int h = threadIdx.x; h < n2 / 2; h += blockDim.x) {
+                const int e = ((h & ~(j - 1)) << 1) | (h & (j - 1)), f = e | j;      // the pair of h in this stage
+                const unsigned long long x = key[e], y = key[f];
+                const bool asc = (e & k) == 0;
+                if ((x > y) == asc) { key[e] = y; key[f] = x; }
             }
-            key[e] = e < m ? (unsigned long long)__double_as_longlong(v) : 0x7ff0000000000000ULL;
+            __syncthreads();
         }
-        if (which == 0) { atomicAdd(&c50, l50); atomicAdd(&ctot, ltot); }
-        __syncthreads();
-        for (int k = 2; k <= n2; k <<= 1)
-            for (int j = k >> 1; j > 0; j >>= 1) {
-                for (int e = threadIdx.x; e < n2; e += blockDim.x) {
-                    const int f = e ^ j;
-                    if (f > e) {
-                        const unsigned long long x = key[e], y = key[f];
-                        const bool asc = (e & k) == 0;
-                        if ((x > y) == asc) { key[e] = y; key[f] = x; }
-                    }
-                }
-                __syncthreads();
-            }
-        if (threadIdx.x == 0) {
-            const double *v = reinterpret_cast<const double *>(key);
-            res[3 * which] = interp_q(v, m, 0.05);
-            res[3 * which + 1] = interp_q(v, m, 0.5);
-            res[3 * which + 2] = interp_q(v, m, 0.95);
-        }
-        __syncthreads();
+    if (threadIdx.x < 3)
+        quant[threadIdx.x] = interp_q(reinterpret_cast<const double *>(key), m,
+                                      threadIdx.x == 0 ? 0.05 : (threadIdx.x == 1 ? 0.5 : 0.95));
+}
+
+// sort_max: the most clones of a pair of the batch that is sorted (at most kSortMax)
+cudaError_t launch_pair_reduce_big(cudaStream_t st, const McPairs &P, int sort_max) {
+    size_t n2 = 1;
+    while (n2 < (size_t)sort_max) n2 <<= 1;
+    const size_t smem = sort_max > 1024 ? n2 * 8 : 0;
+    if (smem > 48 * 1024) {
+        const cudaError_t e = cudaFuncSetAttribute(k_pair_reduce_big, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
     }
-    if (threadIdx.x == 0) {
-        PhResultDev r;
-        r.n = m;
-        r.pad = 0;
-        r.d05 = res[0]; r.d50 = res[1]; r.d95 = res[2];
-        r.t05 = res[3]; r.t50 = res[4]; r.t95 = res[5];
-        r.v05 = res[6]; r.v50 = res[7]; r.v95 = res[8];
-        r.f_r50 = __ddiv_rn((double)c50, (double)m);
-        r.f_rtot = __ddiv_rn((double)ctot, (double)m);
-        *out = r;
-    }
+    k_pair_reduce_big<<<3 * P.n_pairs, kReduceThreads, smem, st>>>(P);
+    return cudaGetLastError();
 }
 
 }  // namespace pgx

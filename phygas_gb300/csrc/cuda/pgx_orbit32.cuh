@@ -161,6 +161,18 @@ struct Acc32 {
     float r2;
 };
 
+// 12^(1 + a) r2^-a'
+template <class M, class Table> PGX_HD F2 halo32_power(const Table &table, F2 r2) {
+    int n = (int)(f32_bits(r2.h) >> 15) - ((127 + kHalo32Lo) << 8);
+    n = n < 0 ? 0 : (n > kHalo32N - 1 ? kHalo32N - 1 : n);
+    const Halo32 T = table(n);
+    const float p = r2.h * T.i, t = p - 1.f, tl = fmaf(r2.l, T.i, fmaf(r2.h, T.i, -p));
+    const float tt = t + tl, w = (tt * tt) * fmaf(tt, fmaf(tt, M::c4, M::c3), M::c2);
+    const float v = M::a1 * t, vl = fmaf(M::a1, tl, fmaf(M::a1l, t, fmaf(M::a1, t, -v))) + w;
+    const float s0 = 1.f + v, s1 = (v - (s0 - 1.f)) + vl;
+    return F2{s0 * T.u0, fmaf(s1, T.u0, fmaf(s0, T.u1, fmaf(s0, T.u2, fmaf(s0, T.u0, -(s0 * T.u0)))))};
+}
+
 // M: the model's lengths as float pairs (bulge_b2(), disk_b2(), disk_a()), the halo's cut-off (cut2 = cut^2, and far() =
 // cut q(cut) for the enclosed mass beyond it) and the series of (1 + t)^-a' (a1 + a1l, c2, c3, c4)
 template <class M, class Table> PGX_HD Acc32 force32(const Force32 &K, const Table &table, F2 x, F2 y, F2 z) {
@@ -169,15 +181,7 @@ template <class M, class Table> PGX_HD Acc32 force32(const Force32 &K, const Tab
     F2 fh;
     if (r2.h < M::cut2) {
         // halo: -K r^-2 / (1 + (12 / r)^(1 + a))
-        int n = (int)(f32_bits(r2.h) >> 15) - ((127 + kHalo32Lo) << 8);
-        n = n < 0 ? 0 : (n > kHalo32N - 1 ? kHalo32N - 1 : n);
-        const Halo32 T = table(n);
-        const float p = r2.h * T.i, t = p - 1.f, tl = fmaf(r2.l, T.i, fmaf(r2.h, T.i, -p));
-        const float tt = t + tl, w = (tt * tt) * fmaf(tt, fmaf(tt, M::c4, M::c3), M::c2);
-        const float v = M::a1 * t, vl = fmaf(M::a1, tl, fmaf(M::a1l, t, fmaf(M::a1, t, -v))) + w;
-        const float s0 = 1.f + v, s1 = (v - (s0 - 1.f)) + vl;
-        const F2 u = {s0 * T.u0,
-                      fmaf(s1, T.u0, fmaf(s0, T.u1, fmaf(s0, T.u2, fmaf(s0, T.u0, -(s0 * T.u0)))))};
+        const F2 u = halo32_power<M>(table, r2);
         const F2 q = f2_rcp(f2_add(f2_mul(ir, u), F2{1.f, 0.f}));
         fh = f2_mul3(f2_mul(f2_sqr(ir), q), K.halo);
     } else {
