@@ -20,40 +20,18 @@
 
 namespace pgx {
 
-// Whether the reference's trace bound (src/phygas.c:379-390: the step's segment m0 -> m1 nowhere nearer than 2 cut
-// tr(M)) rejects a point, from FP32 data: 1 rejects, 0 does not, -1 undecided.  The separations from the split positions
-// are within 3 2^-24 |m| + 10^-12 kpc of the FP64 ones, so the squared distance (a Lipschitz function of the ends) and
-// its evaluation are within 64 2^-24 max(|m0|^2, |m1|^2) + 4 10^-12 kpc^2, and the trace within 10^-5; the FP64
-// comparison's own rounding is far below these margins.
-__device__ __forceinline__ int trace_rejects32(const float (&m0)[3], const float (&m1)[3], float tr, float cut) {
-    const float dx = m1[0] - m0[0], dy = m1[1] - m0[1], dz = m1[2] - m0[2];
-    const float a = fmaf(m0[0], dx, fmaf(m0[1], dy, m0[2] * dz)), dd = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-    const float m00 = fmaf(m0[0], m0[0], fmaf(m0[1], m0[1], m0[2] * m0[2]));
-    const float m11 = fmaf(m1[0], m1[0], fmaf(m1[1], m1[1], m1[2] * m1[2]));
-    const float thr = 2.f * cut * tr, e = fmaf(4e-6f, fmaxf(m00, m11), 4e-12f);
-    // d^2 (or d^2 |dr|^2 with the other side multiplied likewise: nothing is divided)
-    const bool inside = a < 0.f && -a < dd;
-    const float d2 = inside ? fmaf(m00, dd, -a * a) : (a >= 0.f ? m00 : m11), w = inside ? dd : 1.f;
-    if (d2 - e * w > thr * (1.f + 1e-5f) * w) return 1;
-    return d2 + e * w < thr * (1.f - 1e-5f) * w ? 0 : -1;
-}
-
-__device__ __forceinline__ void separation32(const float4 &t0, const float4 &t1, const float4 &c0, const float4 &c1,
-                                             float (&m)[3]) {
-    m[0] = (t0.x - c0.x) + (t0.w - c0.w);
-    m[1] = (t0.y - c0.y) + (t1.x - c1.x);
-    m[2] = (t0.z - c0.z) + (t1.y - c1.y);
-}
-
 // Bound by the FP64 pipe (one warp instruction per 19 cycles and SM).  With a lane walking its own pair, a warp paid for
-// the full point (about 150 FP64 instructions) whenever one lane of 32 needed it, 186 a point on average; the trace test
-// on the FP32 units and full warps for the points that it leaves take 96: 22.9 -> 11.9 ms for 250 stars x 4,087 clusters.  Every value is still the FP64
-// expression; tables without FP32 tracks (one pair of the drop-in API) test in FP64.
+// the full point (about 150 FP64 instructions) whenever one lane of 32 needed it, 186 a point on average: 22.9 ms for
+// 250 stars x 4,087 clusters.  With the trace test on the FP32 units and full warps for the points that it leaves, 11.9;
+// with the points whose form at the point is all (classify32) on their own full warps, 7.8 ms.  Every value is still the
+// FP64 expression; tables without FP32 tracks (one pair of the drop-in API) take the whole of it for every point.
 constexpr int kScan64Warps = 4, kScan64Queue = 64;
 
 __global__ void __launch_bounds__(kScan64Warps * 32) k_scan64(ScreenTables T, double cut, double *__restrict__ chi2T,
                                                               int *__restrict__ kbT, double *__restrict__ sbT) {
-    __shared__ unsigned s_q[kScan64Warps][kScan64Queue];          // owner lane | undecided << 5 | point << 6
+    // two queues: points whose form at the point is all (kPointStart), and the others; owner lane | undecided << 5 |
+    // point << 6
+    __shared__ unsigned s_q[kScan64Warps][2][kScan64Queue];
     __shared__ double s_v[kScan64Warps][32], s_s[kScan64Warps][32];
     __shared__ unsigned s_own[kScan64Warps][32];
     const unsigned all = 0xffffffffu;
@@ -69,47 +47,54 @@ __global__ void __launch_bounds__(kScan64Warps * 32) k_scan64(ScreenTables T, do
         const double R2 = T.R2[c];
         ScanState st;
         st.begin();
-        // the queued points [0, cnt) in FP64, one per lane; then each owner folds its own in queue order, which is
-        // point order
-        auto drain = [&](int cnt) {
+        int qn[2] = {0, 0};
+        // the first cnt points of a queue in FP64, one per lane; then each owner folds its own
+        auto drain = [&](int which, int cnt) {
             __syncwarp();
             s_own[w][lane] = 0u;
             __syncwarp();
             if (lane < cnt) {
-                const unsigned e = s_q[w][lane];
+                const unsigned e = s_q[w][which][lane];
                 const int k = (int)(e >> 6), so = s0 + (int)(e & 31u);
                 const double *tk = T.t64 + (size_t)k * 12 * NT + so, *ck = T.c64 + (size_t)k * 12 * NC + c;
-                double M[6], m0[3], m1[3], sv;
+                double M[6], m0[3], m1[3], sv = 0.0;
 #pragma unroll
                 for (int i = 0; i < 6; i++) M[i] = tk[(6 + i) * NT] + __ldg(ck + (6 + i) * NC);
 #pragma unroll
                 for (int i = 0; i < 3; i++) m0[i] = tk[i * NT] - __ldg(ck + i * NC);
-                const bool more = k + 1 < n;
+                if (which == 0) {
+                    s_v[w][lane] = point_start64(M, R2, m0);
+                } else {
+                    const bool more = k + 1 < n;
 #pragma unroll
-                for (int i = 0; i < 3; i++) m1[i] = more ? tk[(12 + i) * NT] - __ldg(ck + (12 + i) * NC) : m0[i];
-                // a point that the trace bound is known not to reject needs no test: an infinite cut skips it
-                s_v[w][lane] = point_chi2_64(M, R2, m0, m1, more, e & 32u ? cut : kInf, sv);
+                    for (int i = 0; i < 3; i++) m1[i] = more ? tk[(12 + i) * NT] - __ldg(ck + (12 + i) * NC) : m0[i];
+                    s_v[w][lane] = point_chi2_64(M, R2, m0, m1, more, e & 32u ? cut : kInf, sv);
+                }
                 s_s[w][lane] = sv;
                 atomicOr(&s_own[w][e & 31u], 1u << lane);
             }
             __syncwarp();
             for (unsigned mine = s_own[w][lane]; mine; mine &= mine - 1u) {
                 const int j = __ffs(mine) - 1;
-                st.fold((int)(s_q[w][j] >> 6), s_v[w][j], s_s[w][j]);
+                st.fold((int)(s_q[w][which][j] >> 6), s_v[w][j], s_s[w][j]);
             }
             __syncwarp();
+            const int rest = qn[which] - cnt;
+            const unsigned v = lane < rest ? s_q[w][which][cnt + lane] : 0u;
+            __syncwarp();
+            if (lane < rest) s_q[w][which][lane] = v;
+            qn[which] = rest;
         };
-        int qn = 0;
         float4 t0, t1, t2, c0, c1, c2;
         float mc[3], mn[3];
         if (test32) {
             const float4 *a = T.t32 + (size_t)s * 3, *b = T.c32 + (size_t)c * 3;
             t0 = a[0]; t1 = a[1]; t2 = a[2];
             c0 = __ldg(b); c1 = __ldg(b + 1); c2 = __ldg(b + 2);
-            separation32(t0, t1, c0, c1, mc);
+            sep32(t0, t1, c0, c1, mc);
         }
         for (int k = 0; k < n; k++) {
-            int far = -1;
+            int kind = kPointOpen;
             if (test32) {
                 const float tr = (t1.z + c1.z) + (t2.y + c2.y) + (t2.w + c2.w);
                 mn[0] = mc[0]; mn[1] = mc[1]; mn[2] = mc[2];
@@ -117,25 +102,24 @@ __global__ void __launch_bounds__(kScan64Warps * 32) k_scan64(ScreenTables T, do
                     const float4 *a = T.t32 + ((size_t)(k + 1) * NT + s) * 3, *b = T.c32 + ((size_t)(k + 1) * NC + c) * 3;
                     t0 = a[0]; t1 = a[1]; t2 = a[2];
                     c0 = __ldg(b); c1 = __ldg(b + 1); c2 = __ldg(b + 2);
-                    separation32(t0, t1, c0, c1, mn);
+                    sep32(t0, t1, c0, c1, mn);
                 }
-                far = trace_rejects32(mc, mn, tr, cutf);
+                kind = classify32(mc, mn, tr, cutf);
                 mc[0] = mn[0]; mc[1] = mn[1]; mc[2] = mn[2];
             }
-            const bool need = active && far != 1;
-            const unsigned mask = __ballot_sync(all, need);
-            if (need)
-                s_q[w][qn + __popc(mask & ((1u << lane) - 1u))] = (unsigned)lane | (far < 0 ? 32u : 0u) | (unsigned)k << 6;
-            qn += __popc(mask);
-            if (qn >= 32) {
-                drain(32);
-                qn -= 32;
-                const unsigned v = lane < qn ? s_q[w][32 + lane] : 0u;
-                __syncwarp();
-                if (lane < qn) s_q[w][lane] = v;
+            const unsigned entry = (unsigned)lane | (kind == kPointOpen ? 32u : 0u) | (unsigned)k << 6;
+#pragma unroll
+            for (int which = 0; which < 2; which++) {
+                const bool mine = active && (which == 0 ? kind == kPointStart : (kind == kPointNear || kind == kPointOpen));
+                const unsigned m = __ballot_sync(all, mine);
+                if (mine) s_q[w][which][qn[which] + __popc(m & ((1u << lane) - 1u))] = entry;
+                qn[which] += __popc(m);
+                if (qn[which] >= 32) drain(which, 32);
             }
         }
-        if (qn > 0) drain(qn);
+#pragma unroll
+        for (int which = 0; which < 2; which++)
+            if (qn[which] > 0) drain(which, qn[which]);
         if (!active) continue;
         const size_t o = (size_t)c * NT + s;
         chi2T[o] = st.best;

@@ -66,19 +66,77 @@ __device__ __forceinline__ double point_chi2_64(double (&M)[6], double R2, const
     return q;
 }
 
-// running minimum over a pair's points, strict < in point order (the first of equal minima wins)
-struct ScanState {
-    double best, sb;
-    int kb;
-    __device__ __forceinline__ void begin() { best = kInf; sb = 0.0; kb = 0; }
-    __device__ __forceinline__ void point(int k, double (&M)[6], double R2, const double (&m0)[3],
-                                          const double (&m1)[3], bool more, double cut) {
-        double s;
-        const double q = point_chi2_64(M, R2, m0, m1, more, cut, s);
-        fold(k, q, s);
+// The value of a point whose nearest point of the segment is its start (s = 0): the form there, the same operations as
+// point_chi2_64 up to that form -- the second one is the same number and cannot be less.
+__device__ __forceinline__ double point_start64(double (&M)[6], double R2, const double (&m0)[3]) {
+    M[0] += R2; M[3] += R2; M[5] += R2;
+    return Adj64(M).form(m0[0], m0[1], m0[2]);
+}
+
+// What a point's FP64 evaluation has to do, decided from FP32 data wherever its error leaves no doubt.
+//   kPointFar    the reference's trace bound (src/phygas.c:379-390: the step's segment m0 -> m1 nowhere nearer than 2 cut
+//                tr(M)) rejects the point
+//   kPointStart  it does not, and m0.dr > 0: the nearest point of the segment is m0 (point_start64, 60 FP64 operations
+//                where the whole evaluation takes 150)
+//   kPointNear   it does not: no trace test (point_chi2_64 with an infinite cut)
+//   kPointOpen   undecided
+// The separations from the split positions are within 3 2^-24 |m| + 10^-12 kpc of the FP64 ones, so the squared distance
+// (a Lipschitz function of the ends) and its evaluation are within 64 2^-24 max(|m0|^2, |m1|^2) + 4 10^-12 kpc^2, and
+// the trace within 10^-5.  m0.dr is within |m| e + 6 2^-24 |m||dr|, |m| the larger separation and e = 8 2^-24 |m| +
+// 10^-12 kpc the error of dr; twice that decides its sign.  The FP64 arithmetic's own rounding is far below these margins.
+enum { kPointFar, kPointStart, kPointNear, kPointOpen };
+__device__ __forceinline__ int classify32(const float (&m0)[3], const float (&m1)[3], float tr, float cut) {
+    const float eps = 5.9604645e-8f;
+    const float dx = m1[0] - m0[0], dy = m1[1] - m0[1], dz = m1[2] - m0[2];
+    const float a = fmaf(m0[0], dx, fmaf(m0[1], dy, m0[2] * dz)), dd = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+    const float m00 = fmaf(m0[0], m0[0], fmaf(m0[1], m0[1], m0[2] * m0[2]));
+    const float m11 = fmaf(m1[0], m1[0], fmaf(m1[1], m1[1], m1[2] * m1[2]));
+    const float mm = fmaxf(m00, m11), thr = 2.f * cut * tr, e = fmaf(4e-6f, mm, 4e-12f);
+    // d^2 (or d^2 |dr|^2 with the other side multiplied likewise: nothing is divided)
+    const bool inside = a < 0.f && -a < dd;
+    const float d2 = inside ? fmaf(m00, dd, -a * a) : (a >= 0.f ? m00 : m11), w = inside ? dd : 1.f;
+    if (d2 - e * w > thr * (1.f + 1e-5f) * w) return kPointFar;
+    if (!(d2 + e * w < thr * (1.f - 1e-5f) * w)) return kPointOpen;
+    const float big = sqrtf(mm), a_err = big * (fmaf(8.f * eps, big, 1e-12f) + 6.f * eps * sqrtf(dd)) * 1.0001f;
+    return a > 2.f * a_err ? kPointStart : kPointNear;
+}
+
+// separation of star and cluster at one point from the split FP32 positions
+__device__ __forceinline__ void sep32(const float4 &t0, const float4 &t1, const float4 &c0, const float4 &c1,
+                                      float (&m)[3]) {
+    m[0] = (t0.x - c0.x) + (t0.w - c0.w);
+    m[1] = (t0.y - c0.y) + (t1.x - c1.x);
+    m[2] = (t0.z - c0.z) + (t1.y - c1.y);
+}
+
+// classify32 of point k of pair (s, c) with n points, from the FP32 tables (S_c carries the kernel radius there)
+__device__ __forceinline__ int classify_point(const ScreenTables &T, int s, int c, int k, int n, float cut) {
+    const size_t NT = T.nt, NC = T.nc;
+    const float4 *a = T.t32 + ((size_t)k * NT + s) * 3, *b = T.c32 + ((size_t)k * NC + c) * 3;
+    const float4 t0 = a[0], t1 = a[1], t2 = a[2], c0 = __ldg(b), c1 = __ldg(b + 1), c2 = __ldg(b + 2);
+    float m0[3], m1[3];
+    sep32(t0, t1, c0, c1, m0);
+    if (k + 1 < n) {
+        const float4 *p = a + NT * 3, *q = b + NC * 3;
+        sep32(p[0], p[1], __ldg(q), __ldg(q + 1), m1);
+    } else {
+        m1[0] = m0[0]; m1[1] = m0[1]; m1[2] = m0[2];
     }
+    return classify32(m0, m1, (t1.z + c1.z) + (t2.y + c2.y) + (t2.w + c2.w), cut);
+}
+
+// running minimum over a pair's points, in any order: the smallest value, the first point of equal ones (as the
+// reference's strict < finds it in point order).  Doubles >= 0 order as their bit patterns: compared as integers, where a
+// comparison of doubles would take an FP64-pipe slot.  A value that is negative (singular) or NaN is no candidate.
+struct ScanState {
+    static constexpr long long inf = 0x7ff0000000000000LL, minus = (long long)0x8000000000000000ULL;
+    double best, sb;
+    long long key;
+    int kb;
+    __device__ __forceinline__ void begin() { best = kInf; key = inf; sb = 0.0; kb = 0; }
     __device__ __forceinline__ void fold(int k, double q, double s) {
-        if (q >= 0 && q < best) { best = q; kb = k; sb = s; }
+        const long long b = __double_as_longlong(q), v = b & ~minus;
+        if ((b >= 0 || b == minus) && v < inf && (v < key || (v == key && k < kb))) { best = q; key = v; kb = k; sb = s; }
     }
 };
 

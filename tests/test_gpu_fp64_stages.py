@@ -82,3 +82,45 @@ def test_draw_stages_match_the_oracle(built, data):
         checked += 1
         inside += 0 < got[0][0] < 1
     assert checked == 400 and inside > 40, inside
+
+
+@pytest.mark.parametrize("precision", [pg.PGX_FP64, pg.PGX_MIXED], ids=["fp64", "mixed"])
+@pytest.mark.parametrize("cut,r_kernel", [(25.0, 2.0), (4.0, 0.0), (400.0, 8.0)])
+def test_classified_points_give_the_general_paths_bits(built, data, precision, cut, r_kernel):
+    """The points that the FP32 classification rejects or shortens: the batched screens' chi2, argmin and segment fraction
+    against one pair at a time, whose points all take the whole FP64 evaluation, on the same tracks bit for bit."""
+    clusters, stars = data[0][:64], data[1][:20]
+    gpu = dropin._bind(pg.LIB_PATH)
+    C.c_double.in_dll(gpu, "ph_screen_r").value = r_kernel
+    tmax = max(c.tmax_myr for c in clusters)
+    t0, c0 = pg.draw_targets(stars), pg.draw_clusters(clusters)
+    nt = int(np.ceil(tmax / 0.5)) + 1
+    cn = [int(np.ceil(c.tmax_myr / 0.5)) + 1 for c in clusters]
+    with pg.Context(0) as ctx:
+        ctx.set_clusters(clusters, r_kernel=r_kernel, draws=c0)
+        rows = {(int(r["star"]), int(r["cluster"])): r for r in ctx.screen(*t0, tmax, cut, precision)}
+        lins = []
+        for n, ps0, sig in (([nt] * len(t0[0]), t0[0], t0[1]), (cn, c0[0], c0[1])):
+            pos, vel, S = ctx.lin(ps0, sig, n)
+            off = np.concatenate([[0], np.cumsum(n)])
+            out = []
+            for i in range(len(n)):
+                l = dropin.PhLin()
+                l.n = n[i]
+                keep = [np.ascontiguousarray(a[off[i]:off[i + 1]]) for a in (pos, vel, S)]
+                for name, a in zip(("pos", "vel", "S"), keep):
+                    setattr(l, name, C.cast(a.ctypes.data, dict(dropin.PhLin._fields_)[name]))
+                out.append((l, keep))
+            lins.append(out)
+    kept = 0
+    for j in range(len(stars)):
+        for i in range(len(clusters)):
+            kb, sb = C.c_int(), C.c_double()
+            q = gpu.ph_screen_chi2_cut(C.byref(lins[0][j][0]), C.byref(lins[1][i][0]), C.byref(clusters[i]), cut,
+                                       C.byref(kb), C.byref(sb))
+            assert (q < cut) == ((j, i) in rows), (j, i, q)
+            if q < cut:
+                r = rows[(j, i)]
+                assert (r["chi2"], r["kb"], r["sb"]) == (q, kb.value, sb.value), (j, i)
+                kept += 1
+    assert kept > 0
