@@ -401,13 +401,15 @@ __global__ void __launch_bounds__(kScanStars, 6) k_mx_scan32(ScreenTables T, flo
         __syncwarp();
         s_own[w][lane] = 0u;
         __syncwarp();
+        const int e = lane < cnt ? s_q[w][lane] : 0;
+        const float um_own = __shfl_sync(0xffffffffu, um, e & 31);
         if (lane < cnt) {
-            const int e = s_q[w][lane];
             Bound b;
             const bool keep = point_at32(T, s0 + (e & 31), c, e >> 5, cut, b);
-            s_lb[w][lane] = keep ? b.lb : inf;
-            s_ub[w][lane] = keep ? b.ub : inf;
-            atomicOr(&s_own[w][e & 31], 1u << lane);
+            s_lb[w][lane] = b.lb;
+            s_ub[w][lane] = b.ub;
+            // (ub >= lb: a point with lb >= cut or above the min ub changes neither that nor the candidates)
+            if (keep && b.lb < cut && b.lb <= um_own) atomicOr(&s_own[w][e & 31], 1u << lane);
         }
         __syncwarp();
         for (unsigned mine = s_own[w][lane]; mine; mine &= mine - 1u) {
@@ -583,13 +585,15 @@ __global__ void __launch_bounds__(kScanStars, MINB) k_mx_scan32_blocks(const __g
         __syncwarp();
         s_own[w][lane] = 0u;
         __syncwarp();
+        const int e = lane < cnt ? s_q[w][lane] : 0;
+        const float um_own = __shfl_sync(0xffffffffu, um, e & 31);
         if (lane < cnt) {
-            const int e = s_q[w][lane];
             Bound b;
             const bool keep = point_at32_ol(&T, s0 + (e & 31), c, e >> 5, cut, &b);
-            s_lb[w][lane] = keep ? b.lb : inf;
-            s_ub[w][lane] = keep ? b.ub : inf;
-            atomicOr(&s_own[w][e & 31], 1u << lane);
+            s_lb[w][lane] = b.lb;
+            s_ub[w][lane] = b.ub;
+            // (ub >= lb: a point with lb >= cut or above the min ub changes neither that nor the candidates)
+            if (keep && b.lb < cut && b.lb <= um_own) atomicOr(&s_own[w][e & 31], 1u << lane);
         }
         __syncwarp();
         for (unsigned mine = s_own[w][lane]; mine; mine &= mine - 1u) {
