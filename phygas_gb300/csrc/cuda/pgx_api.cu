@@ -297,7 +297,7 @@ int tracks_slot(PgxContext *ctx, int s, double tmax_myr, cudaStream_t st, bool t
     RET(run_lin(ctx, st, nt, k.in_ps0, k.in_sig21, nullptr, ns, k.opos, k.ovel, P<double>(k.t64),
                 P<float4>(k.t32), P<float>(k.tlm), timed, orbit_blocks));
     if (ctx->scan_blocks) {
-        RET(ensure(ctx, k.blk, (size_t)((ns + pgx::kBlockPoints - 1) / pgx::kBlockPoints) * nt * 64));
+        RET(ensure(ctx, k.blk, (size_t)((ns + pgx::kBlockPoints - 1) / pgx::kBlockPoints) * nt * 16 * pgx::kBlkRows));
         MRET(pgx::block_tables(st, nt, ns, nullptr, P<double>(k.t64), P<float>(k.tlm), nullptr, P<float4>(k.blk),
                                ctx->mixed.err));
         ctx->stats.kernels++;

@@ -127,7 +127,10 @@ int mixed_cluster_aux(cudaStream_t st, int nc, int nmax, const int *cn, const do
 // ---- block tables: per object (star or cluster) and block of kBlk points, the data block_skip32 reads --------------
 // t64 [k][12][N] (pos, vel, S), lm [k][N] (FP32 lower bounds on lambda_min(S), with R^2 for the clusters), npts[i]
 // points (nullptr: nmax for every object), R2[i] on the diagonal of S (clusters; nullptr for stars).  Out: blk
-// [b][N][4] float4 = (v, eps) (a, lam) (S0 S1 S2 S3) (S4 S5 lam_lo 0), as pgx_bounds32.cuh describes; a block whose
+// [b][N][4] float4 = (v, eps) (a, lam) (S0 S1 S2 S3) (S4 S5 lam_lo 0), as pgx_bounds32.cuh describes, for clusters, which a
+// warp reads one of; for stars, of which it reads 32 in a row, [b][6][N] with the split position at km in the last two rows
+// (hi, lo_x) (lo_y lo_z 0 0): whole lines where [b][N][4] took four and the position six more (the filter of 2,000 stars 2.66
+// -> 2.60 ms; the points of the walk, each lane at its own star and block, stay in the object's order); a block whose
 // position reference km = kBlk b + kBlk/2 lies past the object's track is zeroed (no pair tests it: a pair tests
 // block b only when km < its point count, which is at most the object's).
 __global__ void k_block_tables(int N, int nmax, const int *__restrict__ npts, const double *__restrict__ t64,
@@ -139,11 +142,13 @@ __global__ void k_block_tables(int N, int nmax, const int *__restrict__ npts, co
     const size_t NN = N;
     const int i = (int)(idx % NN), b = (int)(idx / NN);
     const int n = npts ? npts[i] : nmax;
-    float4 *o = blk + ((size_t)b * NN + i) * 4;
+    const bool rows = R2 == nullptr;
+    float4 *o = rows ? blk + (size_t)b * kBlkRows * NN + i : blk + ((size_t)b * NN + i) * 4;
+    const size_t next = rows ? NN : 1;
     const int km = b * kBlk + kBlk / 2;
     if (km >= n) {
         const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-        o[0] = z; o[1] = z; o[2] = z; o[3] = z;
+        for (int q = 0; q < (rows ? kBlkRows : 4); q++) o[q * next] = z;
         return;
     }
     const int k0 = b * kBlk, ke = min(b * kBlk + kBlk, n - 1);
@@ -289,9 +294,14 @@ __global__ void k_block_tables(int N, int nmax, const int *__restrict__ npts, co
     Sd[0] += r; Sd[3] += r; Sd[5] += r;
     const float lam = __double2float_rd((double)lm[(size_t)ke * NN + i] + (rank1 ? be : delta));
     o[0] = make_float4(v32[0], v32[1], v32[2], __double2float_ru(eps));
-    o[1] = make_float4(a32[0], a32[1], a32[2], lam);
-    o[2] = make_float4((float)Sd[0], (float)Sd[1], (float)Sd[2], (float)Sd[3]);
-    o[3] = make_float4((float)Sd[4], (float)Sd[5], lam_lo, 0.f);
+    o[next] = make_float4(a32[0], a32[1], a32[2], lam);
+    o[2 * next] = make_float4((float)Sd[0], (float)Sd[1], (float)Sd[2], (float)Sd[3]);
+    o[3 * next] = make_float4((float)Sd[4], (float)Sd[5], lam_lo, 0.f);
+    if (rows) {                                                   // split as k_stm_cov splits it
+        const float hx = (float)pm[0], hy = (float)pm[1], hz = (float)pm[2];
+        o[4 * next] = make_float4(hx, hy, hz, (float)(pm[0] - (double)hx));
+        o[5 * next] = make_float4((float)(pm[1] - (double)hy), (float)(pm[2] - (double)hz), 0.f, 0.f);
+    }
 }
 
 int block_tables(cudaStream_t st, int N, int nmax, const int *npts, const double *t64, const float *lm,
@@ -676,7 +686,7 @@ __global__ void __launch_bounds__(kScanStars, MINB) k_mx_scan32_blocks(const __g
             }
         };
         int bn = 0;
-        const float4 *bt = T.blk_t + (size_t)s * 4;
+        const float4 *bt = T.blk_t + s;
         // blocks 0 .. nbt-1 get the test; block nbt, the points after them (fewer than five), is walked untested;
         // the last pass tests nothing and walks what is left (one call site keeps the kernel's code small)
         const int kt = nbt * kBlk, nball = nbt + (kt < n ? 1 : 0);
@@ -684,12 +694,12 @@ __global__ void __launch_bounds__(kScanStars, MINB) k_mx_scan32_blocks(const __g
             bool need = false;
             if (b < nbt && active) {
                 const int km = b * kBlk + kBlk / 2;
-                const float4 *a = bt + (size_t)b * NT * 4, *q = cblk + (size_t)b * cbs;
-                const float4 BT[4] = {a[0], a[1], a[2], a[3]};
+                const float4 *a = bt + (size_t)b * kBlkRows * NT, *q = cblk + (size_t)b * cbs;
+                const float4 BT[4] = {a[0], a[NT], a[2 * NT], a[3 * NT]};
                 const float4 BC[4] = {ldc<STAGE>(q), ldc<STAGE>(q + 1), ldc<STAGE>(q + 2), ldc<STAGE>(q + 3)};
-                const float4 *tm = T.t32 + ((size_t)km * NT + s) * 3, *cm = cc32 + (size_t)km * ccs;
+                const float4 *cm = cc32 + (size_t)km * ccs;
                 float mref[3];
-                sep32(tm[0], tm[1], ldc<STAGE>(cm), ldc<STAGE>(cm + 1), mref);
+                sep32(a[4 * NT], a[5 * NT], ldc<STAGE>(cm), ldc<STAGE>(cm + 1), mref);
                 need = !block_skip32(BT, BC, mref, pair_thr());
             } else if (b < nball) {
                 need = active;
@@ -1531,12 +1541,12 @@ __global__ void k_mx_check_blocks(ScreenTables T, double cut, unsigned long long
     unsigned long long nb_pair = 0;
     for (int b = 0; b < nbt; b++) {
         const int km = b * kBlk + kBlk / 2;
-        const float4 *a = T.blk_t + ((size_t)b * NT + s) * 4, *q = T.blk_c + ((size_t)b * NC + c) * 4;
-        const float4 BT[4] = {a[0], a[1], a[2], a[3]};
+        const float4 *a = T.blk_t + (size_t)b * kBlkRows * NT + s, *q = T.blk_c + ((size_t)b * NC + c) * 4;
+        const float4 BT[4] = {a[0], a[NT], a[2 * NT], a[3 * NT]};
         const float4 BC[4] = {q[0], q[1], q[2], q[3]};
-        const float4 *tm = T.t32 + ((size_t)km * NT + s) * 3, *cm = T.c32 + ((size_t)km * NC + c) * 3;
+        const float4 *cm = T.c32 + ((size_t)km * NC + c) * 3;
         float mref[3];
-        sep32(tm[0], tm[1], cm[0], cm[1], mref);
+        sep32(a[4 * NT], a[5 * NT], cm[0], cm[1], mref);
         k_[0]++;
         nb_pair++;
         const bool settled = block_skip32(BT, BC, mref, (float)cut);

@@ -34,7 +34,8 @@ int gather_columns(cudaStream_t st, int nc, int nmax, const int *order_host, con
 int mixed_cluster_aux(cudaStream_t st, int nc, int nmax, const int *cn, const double *c64, const double *R2,
                       float4 *c32, float *clm, MixedBufs &m);
 // the block tables of N objects' tracks (t64 [k][12][N], lm [k][N], npts[i] points or nmax for all, R2[i] on S's
-// diagonal or none) into blk [ceil(nmax / kBlk)][N][4] float4: what the filter's block test reads
+// diagonal, for clusters) into blk, ceil(nmax / kBlk) blocks of [N][4] float4 or, without R2, of [kBlkRows][N]: what the
+// filter's block test reads
 int block_tables(cudaStream_t st, int N, int nmax, const int *npts, const double *t64, const float *lm,
                  const double *R2, float4 *blk, std::string &err);
 // the draws from the measurement errors on the device (pgx_draws.cu): targets' and clusters' nominal states and
