@@ -59,20 +59,19 @@ FLOPS_PER_PAIR_POINT = 126.0
 # FMA = 2 flops)
 FLOPS_PER_BODY_STEP = 104.0
 FP64_INSTR_PER_BODY_STEP = 36.0 + 3.0 + 29.0
-# the same for one clone-step of the pair Monte Carlo (two body steps, and the FP64 segment test where the FP32 bound
-# does not rule it out), from k_pair_mc_t on the 4,052-pair batch of `bench.py --mode pairs` (200 screen pairs of
-# 2,000 stars + 1 pulsar x 3,852 prefiltered clusters): 73.3 DFMA + 9.3 DADD + 58.9 DMUL executed
-FLOPS_PER_CLONE_STEP = 214.9
-FP64_INSTR_PER_CLONE_STEP = 73.3 + 9.3 + 58.9
+# warp instructions the clone kernel issues per clone-step (two body steps on FP32 pairs and 64-bit integers, and the
+# segment's bound): smsp__inst_executed.sum of k_pair_mc_t on the 4,052-pair batch of `bench.py --mode pairs` (200 screen
+# pairs of 2,000 stars + 1 pulsar x 3,852 prefiltered clusters), 4.16e10 for 1.4905e9 clone-steps, 31.6 lanes active
+CLONE_WARP_INSTR_PER_STEP = 4.15995e10 / 1.4904824e9
 # DRAM traffic of one k_stm_orbits launch on the whole chunk (dram__bytes_read.sum + dram__bytes_write.sum, one ncu
 # capture of `bench.py --mode screen --stars 20000 --parts 1`): 6.7 MB read + 711.9 MB of orbit output written
 ORBIT_TRAFFIC_BYTES = 718.6e6
 # DRAM traffic of the block filter k_mx_scan32_blocks per pair-point (read + write of one ncu capture of one part's
 # launch, `bench.py --mode screen --stars 2500 --parts 1`: 6.30e8 pair-points); a part's launch moves its share
-SCAN_TRAFFIC_PER_PAIR_POINT = (103.69e6 + 47.78e6) / 6.303e8
-# warp instructions the block filter issues per pair-point (smsp__inst_executed.sum of the same capture: 3.57e9 for
+SCAN_TRAFFIC_PER_PAIR_POINT = (103.28e6 + 46.09e6) / 6.303e8
+# warp instructions the block filter issues per pair-point (smsp__inst_executed.sum of the same capture: 2.34e9 for
 # 6.30e8 pair-points); its issue bound is 4 warp instructions per clock per SM (one per scheduler)
-SCAN_WARP_INSTR_PER_PAIR_POINT = 3.5741e9 / 6.303e8
+SCAN_WARP_INSTR_PER_PAIR_POINT = 2.3400e9 / 6.303e8
 ISSUE_PER_CLK_SM = 4
 
 
@@ -280,7 +279,7 @@ def pair_cpu_baseline(cp, pp, n_clones=200, clusters_per_proc=24, procs=None):
                       "slowest process %.1f s" % (procs * k, k, n_clones, clone_steps, max(runs))}
 
 
-def pair_mc_measure(ctx, stars, clusters, cp, rows, want_cpu, fp64_peak):
+def pair_mc_measure(ctx, stars, clusters, cp, rows, want_cpu, clocks):
     """C3-style batch: draws on the host, the autotuner on a sample of it, then the batch timed on the GPU."""
     import numpy as np
     import phygas_gb300 as pg
@@ -339,16 +338,19 @@ def pair_mc_measure(ctx, stars, clusters, cp, rows, want_cpu, fp64_peak):
         ctx.pair_targets(targets_arr, ti, clusters, ci, ncl, 0.05)
         e2e_walls.append(time.perf_counter() - t0)
     rate = cs / (statistics.mean(ms) * 1e-3)
+    import torch
+    issue_peak = (ISSUE_PER_CLK_SM * torch.cuda.get_device_properties(0).multi_processor_count *
+                  (clocks.get("sm_mhz") or clocks.get("sm_max_mhz")) * 1e6)
     out = {"metric": "clone-steps/s", "value": rate, "unit": "clone-steps/s", "ms_per_batch": statistics.mean(ms),
            "workload": "%d screen pairs (p_r50 >= 0.001) + %d pulsars x %d prefiltered clusters; clones U{200,500,1000}, "
                        "dt 0.05 Myr" % (len(take), C3_PULSARS, len(pti)),
            "pairs": int(len(ti)), "clones": int(st["clones"]), "clone_steps": int(cs),
            "launch": "one captured CUDA graph (prep, persistent trace, reduce) per shape, replayed per batch",
-           "roofline": {"bound": "fp64", "kernel": "k_pair_mc_t", "achieved": FLOPS_PER_CLONE_STEP * rate / 1e12,
-                        "peak": fp64_peak / 1e12, "unit": "TFLOP/s", "frac": FLOPS_PER_CLONE_STEP * rate / fp64_peak,
-                        "peak_source": "FP64 FMA probe kernel of this run (pgx_peaks)",
-                        "flops_per_clone_step": FLOPS_PER_CLONE_STEP,
-                        "fp64_instr_frac": FP64_INSTR_PER_CLONE_STEP * rate / (fp64_peak / 2)},
+           "roofline": {"bound": "issue", "kernel": "k_pair_mc_t", "achieved": CLONE_WARP_INSTR_PER_STEP * rate / 1e9,
+                        "peak": issue_peak / 1e9, "unit": "G warp instructions/s",
+                        "frac": CLONE_WARP_INSTR_PER_STEP * rate / issue_peak,
+                        "peak_source": "4 per clock and SM at the SM clock sampled during the timed steps",
+                        "warp_instr_per_clone_step": CLONE_WARP_INSTR_PER_STEP},
            "autotune": {"chosen": {"warps_per_block": table[best][0], "clones_per_lane": table[best][1],
                                    "min_blocks_per_sm": table[best][2]},
                         "ms_on_sample": [{"warps_per_block": w, "clones_per_lane": c, "min_blocks_per_sm": b,
@@ -887,7 +889,7 @@ def main():
     pair_mc = None
     if not args.no_pair:
         try:
-            pair_mc = pair_mc_measure(ctx, stars, clusters, cp, r, rank == 0 and not args.no_cpu, fp64_peak)
+            pair_mc = pair_mc_measure(ctx, stars, clusters, cp, r, rank == 0 and not args.no_cpu, clk.summary())
         except Exception as e:          # reported beside the headline, not part of it
             log("pair Monte Carlo measurement failed: %s" % e)
 

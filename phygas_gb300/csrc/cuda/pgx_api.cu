@@ -51,10 +51,10 @@ constexpr int kSideOrbitBlocksPerSm = 2;
 // with the previous part's screen.  A part's screen must outlast the next part's orbits, whose 2,000 KDK steps set a
 // latency floor of a few ms whatever the part's size, so the first part, whose orbits are exposed, is small and the
 // parts then grow: by default the first of about kPartPairs star-cluster pairs (2,447 stars at 4,087 clusters), each
-// next 1.75 times the last (20,000 stars: 2,447, 4,282, 7,493 and 5,778).  Measured on 20,000 x 4,087: 87.9 ms a
-// step, against 90.1, 88.5, 91.0 and 95.8 ms growing by 1.6, 1.7, 1.8 and 1.9, 89.0 by 1.5, 90.0 in 8 equal parts;
-// beside the screens the orbits take 2 blocks per SM (1 block: 98.7 ms, 3: 89.8).  Earlier, before the block filter:
-// 122 ms whole, 103 in 5 equal parts, 100 in 8, 104 in 12, 116 in 16.
+// next 1.75 times the last (20,000 stars: 2,447, 4,282, 7,493 and 5,778).  Measured on 20,000 x 4,087: 75.9 ms a
+// step, against 79.0 and 82.7 ms growing by 1.5 and 2, 82.8 and 92.8 from 0.8e7 and 1.3e7 pairs; beside the screens the
+// orbits take 2 blocks per SM (1 block: 83.5 ms, 3: 76.2).  With a filter half as slow again: 87.9 ms, and 90.1, 88.5, 91.0
+// and 95.8 growing by 1.6, 1.7, 1.8 and 1.9, 90.0 in 8 equal parts.
 constexpr int kSplitStars = 8192;
 constexpr double kPartPairs = 1.0e7;
 

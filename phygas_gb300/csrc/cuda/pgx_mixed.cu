@@ -11,7 +11,7 @@
 //                    block's points at once (most blocks); the blocks it cannot settle are walked point by point
 //                    as below, 32 blocks at a time on full warps.  The default (PHYGAS_SCAN_BLOCKS=0: k_mx_scan32)
 //   k_mx_scan32      FP32 filter, one thread per pair (warp = 32 stars x one cluster).  Per point: a cheap skip
-//                    test (triangle inequality in the M^-1 norm, one FP32 LDL^T) that settles most points; the rest
+//                    test (the M^-1 norm along the step, one FP32 LDL^T) that settles most points; the rest
 //                    are queued per warp for the bounds LB <= chi2_64 <= UB on the FP64 path's value (the
 //                    reference's trace bound, a Rayleigh lower bound that needs no inversion, and an LDL^T solve
 //                    where it is well conditioned), 32 at a time on full warps.
