@@ -85,7 +85,7 @@ __device__ __forceinline__ double halo_pow_a(double x) {
 __device__ __forceinline__ double rsqrt_h3(double x) {
     const uint32_t hi = f64_hi(x);
     if (!seed_ok(hi)) return rsqrt(x);
-    return rsqrt_refine(x, widen_seed(rsqrtf(seed_arg(hi))));
+    return rsqrt_refine(x, widen_seed(fast_rsqrt(seed_arg(hi))));
 }
 __device__ __forceinline__ double rcp_h3(double d) {
     const uint32_t hi = f64_hi(d);
@@ -171,7 +171,7 @@ __device__ __forceinline__ double quad_accel(double q, int role) {
     const double arg = w + (bulge ? kBulgeB2 : 0.0);
     const uint32_t hi = f64_hi(arg);
     bool ok = seed_ok(hi) && (disk || __double_as_longlong(w) > kTinyR2Bits);
-    const double inv = rsqrt_refine(arg, widen_seed(rsqrtf(seed_arg(hi))));        // ib, iz, ir, ir
+    const double inv = rsqrt_refine(arg, widen_seed(fast_rsqrt(seed_arg(hi))));        // ib, iz, ir, ir
     const double iz = __shfl_sync(all, inv, 1, 4);
     // -GM ib | a + sqrt(z^2 + b^2) | r | r, then ib^2 | D^2 | r / 12 | r / 12
     const double A = fma(inv, bulge ? -kBulgeGM : w, disk ? kDiskA : -0.0);
@@ -188,7 +188,7 @@ __device__ __forceinline__ double quad_accel(double q, int role) {
     const double pow2 = __ldg(&g_halo_pow2[e + kPow2Bias]);
     const double m = __hiloint2double((int)((hB & 0xfffffu) | 0x3ff00000u), __double2loint(B));
     ok = ok && (!disk || seed_ok(hB));
-    const double yD = widen_seed(rsqrtf(seed_arg(hB)));
+    const double yD = widen_seed(fast_rsqrt(seed_arg(hB)));
     //                 disk: 1 / D     halo: x^a, 1 / (1 + p)     helper: ir^2, ir^3, -GM r / 12, c_j^a 2^(a e)
     const double C1 = fma(disk ? yD : (halo ? m : inv), disk ? yD : (halo ? invc : inv), halo ? -1.0 : -0.0);
     const double C2 = fma(C1, disk ? -B : (halo ? c4 : inv), disk ? 1.0 : (halo ? c3 : -0.0));
