@@ -133,6 +133,16 @@ __device__ __forceinline__ void mw_accel(double x, double y, double z, double &a
     az = z * fma(fd * kDiskA, iz, g);
 }
 
+// out of line, for the four-lane step, where it is the rare case (inlined there, 301 stars' orbits took 3.06 ms and not 3.01)
+struct Accel {
+    double x, y, z;
+};
+__device__ __noinline__ Accel mw_accel_any(double x, double y, double z) {
+    Accel a;
+    mw_accel(x, y, z, a.x, a.y, a.z);
+    return a;
+}
+
 // One orbit: position, velocity and the acceleration carried over (one force evaluation per step).
 struct Orbit {
     double x, y, z, vx, vy, vz, ax, ay, az;
@@ -213,9 +223,8 @@ __device__ __forceinline__ double quad_accel(double q, int role) {
     const double g = fma(gb, ib2, fh) + fd;
     double a = q * (halo ? fma(fda, iz, g) : g);
     if (redo) {
-        double ax, ay, az;
-        mw_accel(x, y, z, ax, ay, az);
-        a = bulge ? ax : (disk ? ay : az);
+        const Accel f = mw_accel_any(x, y, z);
+        a = bulge ? f.x : (disk ? f.y : f.z);
     }
     return a;
 }

@@ -93,10 +93,10 @@ static __global__ void __launch_bounds__(32) k_stm_orbits_quad(int N, const doub
 }
 
 // Four lanes per orbit while 7 N orbits at 8 a warp leave each scheduler at most one warp (694 objects on 152 SMs): 1 star
-// 4.7 -> 3.0 ms, 301 stars 4.8 -> 3.1 ms.  Beyond, a scheduler would issue 2 x 32 instructions a step for 16 orbits where
+// 4.7 -> 2.96 ms, 301 stars 4.8 -> 3.01 ms.  Beyond, a scheduler would issue 2 x 32 instructions a step for 16 orbits where
 // one lane per orbit issues 68 for 32.  There, blocks of one warp while the warps are fewer than the schedulers, so that
 // they spread over the SMs (four schedulers share a pipe that serves each at 76 cycles an instruction, three at 64):
-// 2,000 stars 5.3 -> 4.9 ms.  max_blocks > 0: a grid of that many blocks of 128 at most, to run beside other work.
+// 2,000 stars 5.3 -> 4.8 ms.  max_blocks > 0: a grid of that many blocks of 128 at most, to run beside other work.
 cudaError_t launch_stm_orbits(cudaStream_t st, int sms, int N, const double *ps0, const int *npts, int nmax, double *opos,
                               double *ovel, int max_blocks) {
     const long orbits = 7L * N, warps = (orbits + 31) / 32;
