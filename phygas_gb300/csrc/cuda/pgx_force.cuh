@@ -269,7 +269,7 @@ __device__ __forceinline__ int64_t quad_accel32(const F3 &k, float c, int64_t x,
     const F2 iD = f2_rsqrt(f2_add(q, R2)), rc = f2_rcp(a);
     const F2 cube = f2_cube(f2_pick(disk, iD, inv));                                // ib^3 | D^-3 | ir^3
     F2 e = f2_mul3(f2_pick(role >= 2, f2_mul(q, rc), cube), k);                     // bulge | disk | halo
-    if (role >= 2 && !(r2.h < M::cut2)) e = f2_mul3(f2_mul3(cube, k), M::far());
+    if (role >= 2 && !inside_cut<M>(r2)) e = f2_mul3(f2_mul3(cube, k), M::far());
     const F2 ez = f2_mul(e, f2_mul(a, inv));                                        // (disk) along z
     const F2 g1 = f2_add(quad_shfl(e, 2), quad_shfl(e, 0)), fd = quad_shfl(e, 1), fz = quad_shfl(ez, 1);
     return acc_to_fixed(f2_mul(f2_norm(f2_add(g1, f2_pick(role == 2, fz, fd))), f));
