@@ -143,6 +143,19 @@ __device__ __noinline__ Accel mw_accel_any(double x, double y, double z) {
     return a;
 }
 
+// the force of the FP32 orbit's steps near the centre (orbit32_accel), out of line: a few steps of few orbits
+struct MwForce64 {
+    __device__ __forceinline__ void operator()(double x, double y, double z, double *a) const { mw_accel(x, y, z, a[0], a[1], a[2]); }
+};
+__device__ __noinline__ Acc64i mw_accel_near(const OrbitScale s, double dt, int64_t x, int64_t y, int64_t z) {
+    return accel_near(MwForce64(), s, dt, x, y, z);
+}
+struct MwNear {
+    __device__ __forceinline__ Acc64i operator()(const OrbitScale &s, double dt, int64_t x, int64_t y, int64_t z) const {
+        return mw_accel_near(s, dt, x, y, z);
+    }
+};
+
 // One orbit: position, velocity and the acceleration carried over (one force evaluation per step).
 struct Orbit {
     double x, y, z, vx, vy, vz, ax, ay, az;
@@ -273,6 +286,10 @@ __device__ __forceinline__ int64_t quad_accel32(const F3 &k, float c, int64_t x,
     const F2 ez = f2_mul(e, f2_mul(a, inv));                                        // (disk) along z
     const F2 g1 = f2_add(quad_shfl(e, 2), quad_shfl(e, 0)), fd = quad_shfl(e, 1), fz = quad_shfl(ez, 1);
     return acc_to_fixed(f2_mul(f2_norm(f2_add(g1, f2_pick(role == 2, fz, fd))), f));
+}
+// the lane's coordinate of mw_accel_near: quad_accel's bits are mw_accel's (every lane of the warp calls)
+__device__ __noinline__ int64_t quad_accel_near(const OrbitScale s, double dt, int64_t x, int role) {
+    return f64_to_i64(quad_accel((double)x * pow2(s.e - 55), role) * (dt * dt * pow2(61 - s.e + s.k)));
 }
 
 }  // namespace pgx

@@ -343,7 +343,7 @@ __device__ __forceinline__ double norm64(const I3 &v) {
 }
 
 // The segment test of step i (1-based) in FP64: r1, d = r1 - r0 in position units of u kpc, v2 = twice the relative
-// displacement at the step's end in units of u / 64 kpc.  at_r0: the best is at r0 and unevaluated.  r0's distance is
+// displacement at the step's end in units of 2 uv kpc.  at_r0: the best is at r0 and unevaluated.  r0's distance is
 // counted already: only a point beyond it can improve (s > 0).
 //
 // A minimum within a hair of an end of its step: the reference compares the two steps' distances, which differ by less
@@ -353,8 +353,8 @@ __device__ __forceinline__ double norm64(const I3 &v) {
 constexpr double kTie = 0x1p-50;
 enum { kSegNone, kSegBest, kSegAtR0 };
 
-__device__ __noinline__ int segment64(const I3 r1, const I3 d, const I3 v2, int i, double dt, double u, bool at_r0,
-                                      Approach &b, int *tie) {
+__device__ __noinline__ int segment64(const I3 r1, const I3 d, const I3 v2, int i, double dt, double u, double uv,
+                                      bool at_r0, Approach &b, int *tie) {
     const double dx = (double)d.x, dy = (double)d.y, dz = (double)d.z;
     const I3 r0 = r1 - d;
     const double rx = (double)r0.x, ry = (double)r0.y, rz = (double)r0.z;
@@ -369,21 +369,28 @@ __device__ __noinline__ int segment64(const I3 r1, const I3 d, const I3 v2, int 
     *tie = s < 1.0 && (an + dd) * (an + dd) < kTie * dd * m2 ? i + 1 : (hair ? i : 0);
     b.best = dm;
     b.tbest = ((double)(i - 1) + s) * -dt;
-    b.vbest = norm64(v2) * (u * (1.0 / 128.0)) / fabs(dt);
+    b.vbest = norm64(v2) * uv / fabs(dt);
     return kSegBest;
+}
+
+// 2^-55 and 2^-62 kpc in the scale's units: of positions, and half that of displacements
+__device__ __forceinline__ double unit64(const OrbitScale &s) { return pow2(s.e - 55); }
+__device__ __forceinline__ double half_unit64(const OrbitScale &s) { return pow2(s.e - s.k - 62); }
+__device__ __forceinline__ Acc64i mw_accel32(const Force32 &K, const OrbitScale &s, double dt, float near2, long long x,
+                                             long long y, long long z, float &r2) {
+    return orbit32_accel<MwModel32>(K, HaloTable32(), MwNear(), s, dt, near2, x, y, z, r2);
 }
 
 // The record at the end of step i: both orbits there, their displacements those of the next drift
 __device__ __noinline__ Approach vertex64(const Orbit32 a, const Orbit32 b, const Force32 K, const OrbitScale s, int i,
                                           double dt) {
     float r2;
-    const HaloTable32 T;
-    const Acc64i A = accel32<MwModel32>(K, T, s.c, a.x, a.y, a.z, r2), B = accel32<MwModel32>(K, T, s.c, b.x, b.y, b.z, r2);
-    const double u = ldexp(1.0, s.e - 55);
+    const float near2 = orbit32_near2(dt);
+    const Acc64i A = mw_accel32(K, s, dt, near2, a.x, a.y, a.z, r2), B = mw_accel32(K, s, dt, near2, b.x, b.y, b.z, r2);
     const I3 v2 = {2 * (a.wx - b.wx) - (A.x - B.x), 2 * (a.wy - b.wy) - (A.y - B.y),
                    2 * (a.wz - b.wz) - (A.z - B.z)};                 // 2 v dt = 2 w - a dt^2
-    return Approach{norm64(I3{a.x - b.x, a.y - b.y, a.z - b.z}) * u, (double)i * -dt,
-                    norm64(v2) * (u * (1.0 / 128.0)) / fabs(dt)};
+    return Approach{norm64(I3{a.x - b.x, a.y - b.y, a.z - b.z}) * unit64(s), (double)i * -dt,
+                    norm64(v2) * half_unit64(s) / fabs(dt)};
 }
 
 // The closest approach so far, from the float estimates of each step
@@ -404,7 +411,21 @@ struct Near32 {
         tie = 0;
         set_q(s);
     }
-    // a step's dd = d.d, q1 = r1.r1, b1 = r1.d; segment(at_r0) runs segment64 on it, vertex() the record at its start
+    // a step's dd = d.d, q1 = r1.r1, b1 = r1.d, where nothing has to be evaluated: receding with nothing pending, approaching
+    // outside the best, or approaching with a pending record.  false: step() on the same
+    __device__ __forceinline__ bool quick(float dd, float q1, float b1) {
+        const float a0 = b1 - dd;
+        const float t = fminf(dd, q1) > kSureMin ? kSure2 * dd * (q1 + dd) : __int_as_float(0x7f800000);
+        const bool away = a0 > 0.f && a0 * a0 > t, in = !away && b1 < 0.f && b1 * b1 > t;
+        const bool go = in && (pend || q1 * kSureUp < q);
+        if (go) {
+            pend = true;
+            tie = 0;
+            q = q1;
+        }
+        return go || (!pend && (away || (in && !(q1 * kSureDown <= q))));
+    }
+    // segment(at_r0) runs segment64 on it, vertex() the record at its start
     template <class Segment, class Vertex>
     __device__ __forceinline__ void step(float dd, float q1, float b1, const OrbitScale &s, const Segment &segment,
                                          const Vertex &vertex) {
@@ -436,23 +457,53 @@ struct Near32 {
     }
 };
 
-__device__ __forceinline__ double unit64(const OrbitScale &s) { return __hiloint2double((1023 - 55 + s.e) << 20, 0); }
 __device__ __forceinline__ bool in_range32(float ra, float rb, float rmax) {
     return fmaxf(ra, rb) < rmax && fminf(ra, rb) > kOrbit32MinR2;
 }
 
 // the scale of a clone's two orbits (false: none, NaN and infinities included)
-__device__ __forceinline__ bool clone_scale(const double *p, int steps, double dt, OrbitScale &s) {
-    double reach = 0.0, sum = 0.0;
-#pragma unroll
-    for (int o = 0; o < 12; o += 6) {
-        const double x = fmax(fabs(p[o]), fmax(fabs(p[o + 1]), fabs(p[o + 2])));
-        const double v = fmax(fabs(p[o + 3]), fmax(fabs(p[o + 4]), fabs(p[o + 5]))) * fabs(dt);
-        reach = fmax(reach, fmax(2.0 * x + 2.0 * v * steps + 20.0, 256.0 * v));
-    }
+__device__ __forceinline__ bool clone_scale(const double *p, int steps, double dt, float near2, OrbitScale &s) {
+    double va, vb, sum = 0.0;
+    const double ra = orbit32_reach(p, p + 3, steps, dt, va), rb = orbit32_reach(p + 6, p + 9, steps, dt, vb);
 #pragma unroll
     for (int j = 0; j < 12; j++) sum += p[j];                 // fmax passes over NaN
-    return fabs(sum) < 1e300 && orbit32_scale(reach, dt, s);
+    return fabs(sum) < 1e300 && orbit32_start_ok(p, near2) && orbit32_start_ok(p + 6, near2) &&
+           orbit32_units(fmax(ra, rb), fmax(va, vb), dt, s);
+}
+
+// A step that floats alone do not settle: near the centre, or one whose segment or record is evaluated.  Out of line, its data
+// through memory, so that the loop's registers are the common step's (1 x 20,000 clones 2.72 -> 2.53 ms, 300 x 1,000 17.5 -> 16.7).
+struct SlowStep {
+    Orbit32 a, b;            // drifted, not yet kicked
+    I3 sa, sb;               // their drifts
+    Acc64i A, B;             // their accelerations
+    Force32 K;
+    OrbitScale s;
+    Near32 n;
+    float ra, rb, near2, dd, q1, b1;
+    bool done;               // the closest approach needs nothing
+};
+// false: an orbit too close to the centre
+__device__ __noinline__ bool slow_step(SlowStep &t, int i, double dt) {
+    if (t.ra < t.near2) t.A = mw_accel_near(t.s, dt, t.a.x, t.a.y, t.a.z);            // (as orbit32_accel)
+    if (t.rb < t.near2) t.B = mw_accel_near(t.s, dt, t.b.x, t.b.y, t.b.z);
+    if (!(fminf(t.ra, t.rb) > kOrbit32MinR2)) return false;
+    if (t.done) return true;
+    t.n.step(t.dd, t.q1, t.b1, t.s,
+             [&](bool at_r0, Approach &r, int *tie) {
+                 const Orbit32 &a = t.a, &b = t.b;
+                 const I3 v2 = {2 * (a.wx - b.wx) + (t.A.x - t.B.x), 2 * (a.wy - b.wy) + (t.A.y - t.B.y),
+                                2 * (a.wz - b.wz) + (t.A.z - t.B.z)};
+                 return segment64(I3{a.x - b.x, a.y - b.y, a.z - b.z}, t.sa - t.sb, v2, i, dt, unit64(t.s),
+                                  half_unit64(t.s), at_r0, r, tie);
+             },
+             [&]() {
+                 Orbit32 a0 = t.a, b0 = t.b;
+                 a0.x -= t.sa.x; a0.y -= t.sa.y; a0.z -= t.sa.z;
+                 b0.x -= t.sb.x; b0.y -= t.sb.y; b0.z -= t.sb.z;
+                 return vertex64(a0, b0, t.K, t.s, i - 1, dt);
+             });
+    return true;
 }
 
 struct Clone32 {
@@ -460,7 +511,7 @@ struct Clone32 {
     Force32 K;
     OrbitScale s;
     Near32 n;
-    float rmax;              // r2 limit
+    float rmax, near2;       // r2 limits
     bool ok;
     // false: not an orbit for these units (traced in FP64)
     __device__ __forceinline__ bool start(const double *__restrict__ ps, int steps, double dt) {
@@ -469,8 +520,15 @@ struct Clone32 {
         for (int j = 0; j < 12; j++) p[j] = ps[j];
         n.pend = false;
         n.tie = 0;
-        ok = clone_scale(p, steps, dt, s);
-        if (!ok) return false;
+        near2 = orbit32_near2(dt);
+        ok = clone_scale(p, steps, dt, near2, s);
+        if (!ok) {                                            // (stepped along where its lane has another clone)
+            a = b = Orbit32{};
+            K = Force32{};
+            s = OrbitScale{0x1p-23f, 0};
+            rmax = near2 = 0.f;
+            return false;
+        }
         K = force32_constants<MwModel32>(dt, s);
         rmax = orbit32_max_r2(s);
         float ra, rb;
@@ -481,31 +539,28 @@ struct Clone32 {
         return true;
     }
     __device__ __forceinline__ void step(int i, double dt) {
-        const I3 sa = {a.wx >> 6, a.wy >> 6, a.wz >> 6}, sb = {b.wx >> 6, b.wy >> 6, b.wz >> 6};
+        const int sh = 6 + s.k;
+        const I3 sa = {orbit32_drift(a.wx, sh), orbit32_drift(a.wy, sh), orbit32_drift(a.wz, sh)};
+        const I3 sb = {orbit32_drift(b.wx, sh), orbit32_drift(b.wy, sh), orbit32_drift(b.wz, sh)};
         a.x += sa.x; a.y += sa.y; a.z += sa.z;
         b.x += sb.x; b.y += sb.y; b.z += sb.z;
         float ra, rb;
         const HaloTable32 T;
-        const Acc64i A = accel32<MwModel32>(K, T, s.c, a.x, a.y, a.z, ra);
-        const Acc64i B = accel32<MwModel32>(K, T, s.c, b.x, b.y, b.z, rb);
-        ok = ok && in_range32(ra, rb, rmax);
+        Acc64i A = accel32<MwModel32>(K, T, s.c, a.x, a.y, a.z, ra), B = accel32<MwModel32>(K, T, s.c, b.x, b.y, b.z, rb);
         const I3 d = sa - sb, r1 = {a.x - b.x, a.y - b.y, a.z - b.z};
         const float dx = fixed_to_f32(d.x), dy = fixed_to_f32(d.y), dz = fixed_to_f32(d.z);
         const float rx = fixed_to_f32(r1.x), ry = fixed_to_f32(r1.y), rz = fixed_to_f32(r1.z);
-        if (ok)
-            n.step(fmaf(dx, dx, fmaf(dy, dy, dz * dz)), fmaf(rx, rx, fmaf(ry, ry, rz * rz)),
-                   fmaf(rx, dx, fmaf(ry, dy, rz * dz)), s,
-                   [&](bool at_r0, Approach &r, int *tie) {
-                       const I3 v2 = {2 * (a.wx - b.wx) + (A.x - B.x), 2 * (a.wy - b.wy) + (A.y - B.y),
-                                      2 * (a.wz - b.wz) + (A.z - B.z)};
-                       return segment64(r1, d, v2, i, dt, unit64(s), at_r0, r, tie);
-                   },
-                   [&]() {
-                       Orbit32 a0 = a, b0 = b;
-                       a0.x -= sa.x; a0.y -= sa.y; a0.z -= sa.z;
-                       b0.x -= sb.x; b0.y -= sb.y; b0.z -= sb.z;
-                       return vertex64(a0, b0, K, s, i - 1, dt);
-                   });
+        const float dd = fmaf(dx, dx, fmaf(dy, dy, dz * dz)), q1 = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
+        const float b1 = fmaf(rx, dx, fmaf(ry, dy, rz * dz));
+        ok = ok && fmaxf(ra, rb) < rmax;
+        const bool near = fminf(ra, rb) < near2, done = n.quick(dd, q1, b1);
+        if (ok && (near || !done)) {
+            SlowStep t = {a, b, sa, sb, A, B, K, s, n, ra, rb, near2, dd, q1, b1, done};
+            ok = slow_step(t, i, dt);
+            A = t.A;
+            B = t.B;
+            n = t.n;
+        }
         a.wx += A.x; a.wy += A.y; a.wz += A.z;
         b.wx += B.x; b.wy += B.y; b.wz += B.z;
     }
@@ -523,7 +578,7 @@ struct QuadClone32 {
     F3 k;
     OrbitScale s;
     Near32 n;                // alike on the eight lanes
-    float rmax;
+    float rmax, near2;
     bool ok;
     __device__ __forceinline__ static unsigned group() { return 0xffu << (threadIdx.x & 24u); }
     // lanes 0, 1, 2 of the eight hold the target's v, lanes 4, 5, 6 the cluster's: the differences, on every lane
@@ -545,39 +600,53 @@ struct QuadClone32 {
         double p[12];
 #pragma unroll
         for (int j = 0; j < 12; j++) p[j] = ps[j];
-        ok = clone_scale(p, steps, dt, s);
-        if (!ok) s = OrbitScale{0x1p-23f, 0};                 // (traced along with its warp, and again in FP64)
+        near2 = orbit32_near2(dt);
+        ok = clone_scale(p, steps, dt, near2, s);
+        if (!ok) {                                            // (traced along with its warp, and again in FP64)
+            s = OrbitScale{0x1p-23f, 0};
+            near2 = 0.f;
+        }
         k = quad_constant(force32_constants<MwModel32>(ok ? dt : 0.05, s), role);
         rmax = orbit32_max_r2(s);
         const int o = threadIdx.x & 4 ? 6 : 0;
         const double q = role == 0 ? ps[o] : (role == 1 ? ps[o + 1] : ps[o + 2]);
         const double v = role == 0 ? ps[o + 3] : (role == 1 ? ps[o + 4] : ps[o + 5]);
-        x = ok && role < 3 ? f64_to_i64(q * ldexp(1.0, 55 - s.e)) : 0;
+        x = ok && role < 3 ? f64_to_i64(q * pow2(55 - s.e)) : 0;
         float r2;
         const long long a = quad_accel32(k, s.c, x, role, r2);
-        w = (ok && role < 3 ? displacement(v, dt, ldexp(1.0, 61 - s.e)) + a / 2 : 0) + 32;
+        w = (ok && role < 3 ? displacement(v, dt, pow2(61 - s.e + s.k)) + a / 2 : 0) + (32LL << s.k);
         const float rb = __shfl_xor_sync(0xffffffffu, r2, 4);        // (every lane, whatever its ok)
         ok = ok && in_range32(r2, rb, rmax);
         n.start(p, s);
     }
     __device__ __forceinline__ void step(int i, double dt, int role) {
         const unsigned all = 0xffffffffu;
-        const long long sw = w >> 6;
+        const long long sw = orbit32_drift(w, 6 + s.k);
         x += sw;
         float r2;
-        const long long a = quad_accel32(k, s.c, x, role, r2);
+        long long a = quad_accel32(k, s.c, x, role, r2);
         const float rb = __shfl_xor_sync(all, r2, 4);                 // (every lane, whatever its ok)
-        ok = ok && in_range32(r2, rb, rmax);
         const float fd = fixed_to_f32(sw - __shfl_xor_sync(all, sw, 4)), fr = fixed_to_f32(x - __shfl_xor_sync(all, x, 4));
         const float dx = __shfl_sync(all, fd, 0, 8), dy = __shfl_sync(all, fd, 1, 8), dz = __shfl_sync(all, fd, 2, 8);
         const float rx = __shfl_sync(all, fr, 0, 8), ry = __shfl_sync(all, fr, 1, 8), rz = __shfl_sync(all, fr, 2, 8);
-        if (ok)
-            n.step(fmaf(dx, dx, fmaf(dy, dy, dz * dz)), fmaf(rx, rx, fmaf(ry, ry, rz * rz)),
-                   fmaf(rx, dx, fmaf(ry, dy, rz * dz)), s,
-                   [&](bool at_r0, Approach &r, int *tie) {
-                       return segment64(diff3(x), diff3(sw), diff3(2 * w + a), i, dt, unit64(s), at_r0, r, tie);
-                   },
-                   [&]() { return vertex(x - sw, i - 1, dt); });
+        const float dd = fmaf(dx, dx, fmaf(dy, dy, dz * dz)), q1 = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
+        const float b1 = fmaf(rx, dx, fmaf(ry, dy, rz * dz));
+        ok = ok && fmaxf(r2, rb) < rmax;
+        const bool near = fminf(r2, rb) < near2, done = n.quick(dd, q1, b1);
+        if (__any_sync(all, ok && (near || !done))) {
+            if (__any_sync(all, ok && near)) {                        // (as orbit32_accel)
+                const long long m = quad_accel_near(s, dt, x, role);
+                if (ok && r2 < near2) a = m;
+                ok = ok && fminf(r2, rb) > kOrbit32MinR2;
+            }
+            if (ok && !done)
+                n.step(dd, q1, b1, s,
+                       [&](bool at_r0, Approach &r, int *tie) {
+                           return segment64(diff3(x), diff3(sw), diff3(2 * w + a), i, dt, unit64(s), half_unit64(s), at_r0,
+                                            r, tie);
+                       },
+                       [&]() { return vertex(x - sw, i - 1, dt); });
+        }
         w += a;
     }
     __device__ __forceinline__ void finish(int steps, double dt) {
@@ -605,22 +674,31 @@ static __global__ void __launch_bounds__(32) k_coarse_tracks(int N, const double
 #pragma unroll
     for (int j = 0; j < 6; j++) p12[j] = p12[6 + j] = q[j];
     OrbitScale s;
-    bool ok = clone_scale(p12, (n - 1) * kSub, dt, s);
-    if (!ok) s = OrbitScale{0x1p-23f, 0};
+    float near2 = orbit32_near2(dt);
+    bool ok = clone_scale(p12, (n - 1) * kSub, dt, near2, s);
+    if (!ok) {
+        s = OrbitScale{0x1p-23f, 0};
+        near2 = 0.f;
+    }
     const F3 k = quad_constant(force32_constants<MwModel32>(dt, s), role);
     const float rmax = orbit32_max_r2(s);
     const double unit = unit64(s);
-    long long x = ok && role < 3 ? f64_to_i64(q[c] * ldexp(1.0, 55 - s.e)) : 0;
+    long long x = ok && role < 3 ? f64_to_i64(q[c] * pow2(55 - s.e)) : 0;
     float r2;
     const long long a0 = quad_accel32(k, s.c, x, role, r2);
     ok = ok && in_range32(r2, r2, rmax);
-    long long w = (ok && role < 3 ? displacement(q[3 + c], dt, ldexp(1.0, 61 - s.e)) + a0 / 2 : 0) + 32;
+    long long w = (ok && role < 3 ? displacement(q[3 + c], dt, pow2(61 - s.e + s.k)) + a0 / 2 : 0) + (32LL << s.k);
     for (int j = 0; j < nw; j++) {
         if (j > 0) {
 #pragma unroll 1
             for (int m = 0; m < kSub; m++) {
-                x += w >> 6;
-                w += quad_accel32(k, s.c, x, role, r2);
+                x += orbit32_drift(w, 6 + s.k);
+                long long a = quad_accel32(k, s.c, x, role, r2);
+                if (__any_sync(all, r2 < near2)) {                    // (as orbit32_accel)
+                    const long long f = quad_accel_near(s, dt, x, role);
+                    if (r2 < near2) a = f;
+                }
+                w += a;
                 ok = ok && (j >= n || in_range32(r2, r2, rmax));
             }
         }

@@ -10,12 +10,17 @@
 //  * the force is evaluated on pairs of floats (value = h + l, about 48 bits), each product and sum with its rounding
 //    error carried along by fused multiply-adds; the constants are the FP64 ones, in three floats.
 // The force's error, 2^-47.8 relative (rms) and random, enters w through a dt^2 ~ 2^-11 w, below FP64's own rounding
-// of the velocity.  Against 113-bit arithmetic over 100 Myr (2,000 steps) the position is off by 1.4e-14 kpc rms where
-// the FP64 step is off by 7.6e-14, and by the FP64 step's 7e-14 on orbits inside 1 kpc (tests/test_orbit32.py).
+// of the velocity -- where an orbit turns slowly.  Within kOrbit32Near |dt| of the centre a dt is so large a part of v that
+// it is not: there the force is FP64's (orbit32_accel).
 //
-// Orbits larger than 256 kpc take units 2^e times larger (OrbitScale).  Valid for 0.01 <= |dt| <= 0.125 Myr and r >
-// 2^-10 kpc; a caller traces other orbits in FP64.  Below 0.01 Myr the displacement's unit would be coarser than
-// FP64's rounding of the velocity, above 0.125 Myr a dt^2 could pass its integer's range.
+// What is traced this way is what comes out no further from exact arithmetic than FP64 steps, measured against 113-bit
+// arithmetic (tests/test_orbit32_range.py): 0.01 <= |dt| <= 0.125 Myr, a start outside kOrbit32Near |dt| and 0.4 kpc, and a reach of
+// less than 2,048 kpc.  2,000 steps of 0.05 Myr at 8 kpc: 1.3e-14 kpc rms, the FP64 step 8e-14; at 1 kpc 2e-14 and 7e-14;
+// at 1,024 kpc 1.6e-13 and 1.7e-12.  Beyond, and with less than 2^-10 kpc to the centre, a caller traces in FP64.
+//
+// The units.  Orbits larger than 256 kpc take units 2^e times larger; steps of 1/16 Myr and less take displacements 2^k
+// times finer, which FP64's rounding of a slow orbit's velocity asks for (OrbitScale).  FP64 rounds a position at 2,048 kpc
+// to 2^-42 kpc, 2^10 times this unit there; at 30,000 kpc and steps of 0.01 Myr a displacement's unit was the larger error.
 #pragma once
 #include <cstdint>
 #include "pgx_bits.cuh"
@@ -122,14 +127,30 @@ PGX_HD int32_t f32_rint(float x) {
 #endif
 }
 
+// 2^n, normal
+PGX_HD double pow2(int n) {
+#ifdef __CUDA_ARCH__
+    return __hiloint2double((1023 + n) << 20, 0);
+#else
+    return ldexp(1.0, n);
+#endif
+}
+
 // ---- units -------------------------------------------------------------------------------------------------------
-// 2^e times 2^-55 kpc (positions) and 2^-61 kpc (displacements): c = 2^(e - 23) kpc, the unit of a position's high word
+// 2^e times 2^-55 kpc (positions) and 2^-(61 + k) kpc (displacements): c = 2^(e - 23) kpc, the unit of a position's high
+// word
 struct OrbitScale {
     float c;
-    int e;
+    int e, k = 0;
 };
-constexpr double kOrbit32MinDt = 0.01, kOrbit32MaxDt = 0.125, kOrbit32MaxReach = 1e6;
+constexpr double kOrbit32MinDt = 0.01, kOrbit32MaxDt = 0.125, kOrbit32MaxReach = 2048.0;
+constexpr double kOrbit32Near = 14.0, kOrbit32MinStart = 0.4;      // kpc per Myr of step; kpc
 constexpr float kOrbit32MinR2 = 0x1p-20f;
+
+PGX_HD float orbit32_near2(double dt) {
+    const double r = kOrbit32Near * dt;
+    return (float)(r * r);
+}
 
 // The scale for orbits that reach at most `reach` kpc; false: trace them in FP64 (NaN included).
 PGX_HD bool orbit32_scale(double reach, double dt, OrbitScale &s) {
@@ -140,24 +161,43 @@ PGX_HD bool orbit32_scale(double reach, double dt, OrbitScale &s) {
     for (double lim = 256.0; lim <= reach; lim *= 2.0) { s.e++; s.c *= 2.f; }
     return true;
 }
+// The scale with the displacements' own unit: k = 2 for steps of 1/16 Myr and less, 3 from 1/32, 4 from 1/64, and e more, so
+// that a larger orbit's displacements stay as fine -- less where v dt would leave a quarter of the integer's range
+PGX_HD bool orbit32_units(double reach, double vdt, double dt, OrbitScale &s) {
+    if (!orbit32_scale(reach, dt, s)) return false;
+    const double d = fabs(dt);
+    s.k = s.e + (d <= 0.015625 ? 4 : (d <= 0.03125 ? 3 : (d <= 0.0625 ? 2 : 0)));
+    while (s.k > 0 && vdt >= pow2(s.e - s.k - 1)) s.k--;
+    return vdt < pow2(s.e - s.k - 1);
+}
+// The reach to ask for an orbit from q, v over `steps` steps: twice the straight line's, but under 0.4 kpc/Myr within 20 kpc
+// an orbit is bound and stays inside 200 kpc (one that does not is noticed: orbit32_max_r2)
+PGX_HD double orbit32_reach(const double *q, const double *v, double steps, double dt, double &vdt) {
+    const double x = fmax(fabs(q[0]), fmax(fabs(q[1]), fabs(q[2])));
+    const double u = fmax(fabs(v[0]), fmax(fabs(v[1]), fabs(v[2])));
+    vdt = u * fabs(dt);
+    double drift = 2.0 * vdt * steps;
+    if (u < 0.4 && x < 20.0) drift = fmin(drift, 200.0);
+    return fmax(2.0 * x + drift + 20.0, 512.0 * vdt);
+}
 // r2 below this: inside the positions' range
 PGX_HD float orbit32_max_r2(const OrbitScale &s) { return (s.c * 0x1p31f) * (s.c * 0x1p31f) * 0.98f; }
 
-// the model's GM times dt^2 2^37 in the scale's units (a dt^2's high part is an integer multiple of 2^-37, the rest of
-// 2^-61)
+// the model's GM times dt^2 2^(37 + k) in the scale's units (a dt^2's high part is an integer multiple of 2^-(37 + k), the
+// rest of 2^-(61 + k))
 struct Force32 {
     F3 bulge, disk, halo;
 };
 // M: the model's FP64 constants
 template <class M> PGX_HD Force32 force32_constants(double dt, const OrbitScale &s) {
-    const double u = ldexp(1.0, 37 - s.e), h = M::halo_GM * M::halo_inv_a;
+    const double u = pow2(37 - s.e + s.k), h = M::halo_GM * M::halo_inv_a;
     Force32 k = {split3_square(-M::bulge_GM, dt, u), split3_square(-M::disk_GM, dt, u), split3_square(-h, dt, u)};
     k.halo.c -= (float)(fma(M::halo_GM, M::halo_inv_a, -h) * dt * dt * u);
     return k;
 }
 
 struct Acc32 {
-    F2 x, y, z;          // a dt^2 2^37 in the scale's units
+    F2 x, y, z;          // a dt^2 2^(37 + k) in the scale's units
     float r2;
 };
 
@@ -212,8 +252,8 @@ PGX_HD F2 fixed_to_f2(int64_t X, float c) {
     const float mid = (float)(int32_t)((d << 24) | (lo >> 8)), s = fmaf(mid, c1, high);
     return F2{s, fmaf((float)(int32_t)(lo & 0xffu), c * 0x1p-32f, fmaf(mid, c1, high - s))};
 }
-// a dt^2 2^37 as an integer in units of 2^-61 kpc.  |a| < 0.18 kpc/Myr^2 anywhere in this model, so with |dt| <= 0.125
-// |a.h| < 2^28.6 and, the force's factors being normalized, |a.l| < 3 2^-24 |a.h|: both integers fit 32 bits.
+// a dt^2 2^(37 + k) as an integer in units of 2^-(61 + k) kpc.  |a| < 0.18 kpc/Myr^2 anywhere in this model, so with
+// |dt| <= 0.125 and k of its step |a.h| < 2^28.6 and, the force's factors being normalized, |a.l| < 3 2^-24 |a.h|: both integers fit 32 bits.
 PGX_HD int64_t acc_to_fixed(F2 a) {
     const int32_t n = f32_rint(a.h);
     const int32_t m = f32_rint(((a.h - (float)n) + a.l) * 0x1p24f);
@@ -221,20 +261,13 @@ PGX_HD int64_t acc_to_fixed(F2 a) {
 }
 
 // One orbit: position and the coming drift's displacement, the latter with half a position unit added once so that
-// the drift's shift rounds to nearest.
+// the drift's shift (by 6 + k) rounds to nearest.
 struct Orbit32 {
     int64_t x, y, z, wx, wy, wz;
 };
 struct Acc64i {
     int64_t x, y, z;     // a dt^2 in displacement units
 };
-
-template <class M, class Table>
-PGX_HD Acc64i accel32(const Force32 &K, const Table &table, float c, int64_t x, int64_t y, int64_t z, float &r2) {
-    const Acc32 a = force32<M>(K, table, fixed_to_f2(x, c), fixed_to_f2(y, c), fixed_to_f2(z, c));
-    r2 = a.r2;
-    return Acc64i{acc_to_fixed(a.x), acc_to_fixed(a.y), acc_to_fixed(a.z)};
-}
 
 PGX_HD int64_t f64_to_i64(double x) {
 #ifdef __CUDA_ARCH__
@@ -243,22 +276,61 @@ PGX_HD int64_t f64_to_i64(double x) {
     return (int64_t)llrint(x);
 #endif
 }
+template <class M, class Table>
+PGX_HD Acc64i accel32(const Force32 &K, const Table &table, float c, int64_t x, int64_t y, int64_t z, float &r2) {
+    const Acc32 a = force32<M>(K, table, fixed_to_f2(x, c), fixed_to_f2(y, c), fixed_to_f2(z, c));
+    r2 = a.r2;
+    return Acc64i{acc_to_fixed(a.x), acc_to_fixed(a.y), acc_to_fixed(a.z)};
+}
+
+// The force of a step that ends near the centre in FP64: force(x, y, z, a) gives a in kpc/Myr^2 at a position in kpc
+template <class F>
+PGX_HD Acc64i accel_near(const F &force, const OrbitScale &s, double dt, int64_t x, int64_t y, int64_t z) {
+    const double u = pow2(s.e - 55), w = dt * dt * pow2(61 - s.e + s.k);
+    double a[3];
+    force((double)x * u, (double)y * u, (double)z * u, a);
+    return Acc64i{f64_to_i64(a[0] * w), f64_to_i64(a[1] * w), f64_to_i64(a[2] * w)};
+}
+// a step's force: on pairs of floats, within near2 = orbit32_near2(dt) near's (accel_near)
+template <class M, class Table, class Near>
+PGX_HD Acc64i orbit32_accel(const Force32 &K, const Table &table, const Near &near, const OrbitScale &s, double dt, float near2,
+                            int64_t x, int64_t y, int64_t z, float &r2) {
+    Acc64i a = accel32<M>(K, table, s.c, x, y, z, r2);
+    if (r2 < near2) a = near(s, dt, x, y, z);
+    return a;
+}
+
 // v dt in displacement units, the product's rounding included
 PGX_HD int64_t displacement(double v, double dt, double unit) {
     const double w = v * dt;
     return f64_to_i64(w * unit) + f64_to_i64(fma(v, dt, -w) * unit);
 }
+// whether an orbit may start at q: outside the near field, and where FP64's positions are no finer than the unit's
+PGX_HD bool orbit32_start_ok(const double *q, float near2) {
+    return fma(q[0], q[0], fma(q[1], q[1], q[2] * q[2])) >= fmax((double)near2, kOrbit32MinStart * kOrbit32MinStart);
+}
+// a displacement's drift in position units, sh = 6 + k
+PGX_HD int64_t orbit32_drift(int64_t w, int sh) {
+#ifdef __CUDA_ARCH__
+    const int hi = (int)(w >> 32);
+    return (int64_t)(hi >> sh) << 32 | __funnelshift_r((unsigned)w, (unsigned)hi, sh);
+#else
+    return w >> sh;
+#endif
+}
+
 // position q and velocity v (kpc, kpc/Myr): displacements of the first drift, v dt + a dt^2 / 2; |q| and |v dt| below the
-// scale's range
+// scale's range, q outside the near field
 template <class M, class Table>
 PGX_HD void orbit32_start(Orbit32 &o, const Force32 &K, const Table &table, const OrbitScale &s, const double *q,
                           const double *v, double dt, float &r2) {
-    const double ux = ldexp(1.0, 55 - s.e), uw = ldexp(1.0, 61 - s.e);
+    const double ux = pow2(55 - s.e), uw = pow2(61 - s.e + s.k);
+    const int64_t half = 32LL << s.k;
     o.x = f64_to_i64(q[0] * ux); o.y = f64_to_i64(q[1] * ux); o.z = f64_to_i64(q[2] * ux);
     const Acc64i a = accel32<M>(K, table, s.c, o.x, o.y, o.z, r2);
-    o.wx = displacement(v[0], dt, uw) + a.x / 2 + 32;
-    o.wy = displacement(v[1], dt, uw) + a.y / 2 + 32;
-    o.wz = displacement(v[2], dt, uw) + a.z / 2 + 32;
+    o.wx = displacement(v[0], dt, uw) + a.x / 2 + half;
+    o.wy = displacement(v[1], dt, uw) + a.y / 2 + half;
+    o.wz = displacement(v[2], dt, uw) + a.z / 2 + half;
 }
 
 }  // namespace pgx
