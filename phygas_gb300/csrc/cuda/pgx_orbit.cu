@@ -283,11 +283,11 @@ __device__ __noinline__ Approach trace_clone64(const double *__restrict__ ps, in
     return Approach{n.best, n.tbest, n.vbest};
 }
 
-// One clone by a whole warp in FP64 (the same bits): lanes 0-3 trace its target, 4-7 its cluster (quad_accel), the
-// others repeat them.  A step takes 32 FP64 instructions where trace_clone64 takes 136, so a warp with one or two
-// such clones ends four times sooner.
-__device__ __noinline__ Approach trace_clone64_warp(const double *__restrict__ ps, int steps, double dt) {
-    const unsigned all = 0xffffffffu;
+// Four clones by a warp in FP64, eight lanes each (the same bits): lanes 0-3 of the eight trace the target, 4-7 the cluster
+// (quad_accel).  ps, steps and dt are the eight's clone's; every lane of the warp calls.  A step takes 32 FP64 instructions
+// where trace_clone64 takes 136, so up to three such passes end sooner.
+__device__ __noinline__ Approach trace_clone64_eights(const double *__restrict__ ps, int steps, double dt) {
+    const unsigned all = 0xffffffffu, eight = 0xffu << (threadIdx.x & 24u);
     const int role = threadIdx.x & 3, c = role < 3 ? role : 2;
     const double *p = ps + (threadIdx.x & 4 ? 6 : 0);
     QuadOrbit o;
@@ -295,17 +295,21 @@ __device__ __noinline__ Approach trace_clone64_warp(const double *__restrict__ p
     o.v = role < 3 ? p[3 + c] : 0.0;
     o.init(role);
     Nearest n;
-    // component k of the target's orbit less the cluster's, on every lane
-    auto diff = [&](double v, int k) { return __shfl_sync(all, v, k) - __shfl_sync(all, v, 4 + k); };
-    n.start(diff(o.q, 0), diff(o.q, 1), diff(o.q, 2), diff(o.v, 0), diff(o.v, 1), diff(o.v, 2));
+    // component k of the target's orbit less the cluster's, on each of the lanes m (the warp's, or one eight's)
+    auto diff = [&](unsigned m, double v, int k) { return __shfl_sync(m, v, k, 8) - __shfl_sync(m, v, 4 + k, 8); };
+    n.start(diff(all, o.q, 0), diff(all, o.q, 1), diff(all, o.q, 2), diff(all, o.v, 0), diff(all, o.v, 1),
+            diff(all, o.v, 2));
     const double h = 0.5 * dt;
+    const int most = __reduce_max_sync(all, steps);
 #pragma unroll 1
-    for (int i = 1; i <= steps; i++) {
+    for (int i = 1; i <= most; i++) {
         o.kdk(dt, h, role);
-        n.segment(i, dt, diff(o.q, 0), diff(o.q, 1), diff(o.q, 2), [&]() {
-            const double wx = diff(o.v, 0), wy = diff(o.v, 1), wz = diff(o.v, 2);
-            return sqrt(fma(wx, wx, fma(wy, wy, wz * wz)));
-        });
+        const double x = diff(all, o.q, 0), y = diff(all, o.q, 1), z = diff(all, o.q, 2);
+        if (i <= steps)
+            n.segment(i, dt, x, y, z, [&]() {
+                const double wx = diff(eight, o.v, 0), wy = diff(eight, o.v, 1), wz = diff(eight, o.v, 2);
+                return sqrt(fma(wx, wx, fma(wy, wy, wz * wz)));
+            });
     }
     return Approach{n.best, n.tbest, n.vbest};
 }
@@ -724,22 +728,33 @@ cudaError_t launch_coarse_tracks(cudaStream_t st, int N, const double *ps, const
     return cudaGetLastError();
 }
 
-// The clones of a warp that take the FP64 trace: n steps of each lane's clone (0: none; every lane calls).  A few are
-// traced by the whole warp one after the other, more (a step length or a reach outside the FP32 orbit's) lane by lane:
-// 4 x 32 instructions against 136.
+// The clones of a warp that take the FP64 trace: n steps of each lane's clone (0: none; every lane calls).  Up to twelve are
+// traced four at a time (3 x 32 FP64 instructions a step at most), more lane by lane (136).  One after the other, as it was,
+// 10 pairs x 400 clones at steps of 0.2 Myr took 8.5 ms, four at a time 2.3.
 __device__ __forceinline__ void trace_fp64(const double *ps, int n, int steps, double dt, Approach &r) {
     const unsigned all = 0xffffffffu;
     unsigned m = __ballot_sync(all, n > 0);
-    if (__popc(m) > 4) {
+    if (__popc(m) > 12) {
         if (n > 0) r = trace_clone64(ps, min(n, steps), dt);
         return;
     }
-    for (; m; m &= m - 1u) {
-        const int l = __ffs(m) - 1;
-        const unsigned long long p = __shfl_sync(all, (unsigned long long)ps, l);
-        const Approach x = trace_clone64_warp((const double *)p, __shfl_sync(all, min(n, steps), l),
-                                              __shfl_sync(all, dt, l));
-        if ((int)(threadIdx.x & 31) == l) r = x;
+    const int lane = threadIdx.x & 31;
+    while (m) {
+        // the eights take the next four set lanes' clones (with fewer left, the others repeat the first)
+        int src = __ffs(m) - 1;
+        unsigned left = m;
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            if (k == lane >> 3 && left) src = __ffs(left) - 1;
+            left &= left - 1u;
+        }
+        const unsigned long long p = __shfl_sync(all, (unsigned long long)ps, src);
+        const Approach x = trace_clone64_eights((const double *)p, __shfl_sync(all, min(n, steps), src),
+                                                __shfl_sync(all, dt, src));
+        const int k = __popc(m & ((1u << lane) - 1u)), from = 8 * min(k, 3);
+        const Approach y = {__shfl_sync(all, x.best, from), __shfl_sync(all, x.tbest, from), __shfl_sync(all, x.vbest, from)};
+        if ((m >> lane & 1u) && k < 4) r = y;
+        m = left;
     }
 }
 
