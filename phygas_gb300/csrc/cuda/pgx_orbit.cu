@@ -1210,11 +1210,7 @@ __global__ void __launch_bounds__(kReduceThreads) k_pair_reduce_big(McPairs P) {
 cudaError_t launch_pair_reduce_big(cudaStream_t st, const McPairs &P, int sort_max) {
     size_t n2 = 1;
     while (n2 < (size_t)sort_max) n2 <<= 1;
-    const size_t smem = sort_max > 1024 ? n2 * 8 : 0;
-    if (smem > 48 * 1024) {
-        const cudaError_t e = cudaFuncSetAttribute(k_pair_reduce_big, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-    }
+    const size_t smem = sort_max > 1024 ? n2 * 8 : 0;         // (allowed for up to kSortMax clones by orbit_setup)
     k_pair_reduce_big<<<3 * P.n_pairs, kReduceThreads, smem, st>>>(P);
     return cudaGetLastError();
 }
@@ -1418,7 +1414,8 @@ extern "C" int pgx_pair_noalloc(void *stream, int n_pairs, int n_clones, const i
 
 namespace pgx {
 // The halo power tables of pgx_force.cuh, filled once per device (before the first orbit kernel on it; call it
-// outside any stream capture).
+// outside any stream capture), and the shared memory k_pair_reduce_big may ask for: a limit of the function on the device,
+// for every context and thread, so it is set to the most once and not to each launch's own.
 int orbit_setup(int dev) {
     static std::mutex mu;
     static bool ready[64] = {};
@@ -1432,6 +1429,8 @@ int orbit_setup(int dev) {
     k_halo_tables<<<1, kHaloTableThreads>>>();
     k_halo32_table<<<(kHalo32N + 255) / 256, 256>>>();
     cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_pair_reduce_big, cudaFuncAttributeMaxDynamicSharedMemorySize, kSortMax * 8);
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
     if (e != cudaSuccess) return 2;
     ready[dev] = true;
