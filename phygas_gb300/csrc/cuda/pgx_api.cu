@@ -577,7 +577,7 @@ int pgx_draw_pair_batch_gpu(PgxContext *ctx, int n_pairs, const PhTarget *t, con
     auto pad = [](size_t b) { return (b + 15) & ~(size_t)15; };
     const size_t bt = pad((size_t)nt * sizeof(PhTarget)), bc = pad((size_t)nc * sizeof(PhCluster));
     const size_t bi = pad((size_t)(n_pairs + 1) * 4), b8 = pad((size_t)n_pairs * 8);
-    RET(ensure(ctx, ctx->x_draw, bt + bc + 5 * bi + 2 * b8 + pgx::pair_frames_bytes(n_pairs) + pad((size_t)cap * 4)));
+    RET(ensure(ctx, ctx->x_draw, bt + bc + 5 * bi + 2 * b8 + pgx::pair_frames_bytes(n_pairs) + pad((size_t)cap * 8)));
     char *b = P<char>(ctx->x_draw);
     auto take = [&](size_t bytes) { char *p = b; b += bytes; return p; };
     PhTarget *d_t = (PhTarget *)take(bt);
@@ -587,7 +587,7 @@ int pgx_draw_pair_batch_gpu(PgxContext *ctx, int n_pairs, const PhTarget *t, con
     uint64_t *d_seed = (uint64_t *)take(b8);
     long long *d_slot = (long long *)take(b8);
     void *d_frames = take(pgx::pair_frames_bytes(n_pairs));
-    int *d_gi = (int *)take(0);
+    uint64_t *d_at = (uint64_t *)take(0);
     CK(cudaMemcpyAsync(d_t, t, (size_t)nt * sizeof(PhTarget), cudaMemcpyHostToDevice, ctx->st));
     CK(cudaMemcpyAsync(d_c, c, (size_t)nc * sizeof(PhCluster), cudaMemcpyHostToDevice, ctx->st));
     CK(cudaMemcpyAsync(d_ti, ti, (size_t)n_pairs * 4, cudaMemcpyHostToDevice, ctx->st));
@@ -597,7 +597,7 @@ int pgx_draw_pair_batch_gpu(PgxContext *ctx, int n_pairs, const PhTarget *t, con
     CK(cudaMemcpyAsync(d_slot, slot.data(), (size_t)n_pairs * 8, cudaMemcpyHostToDevice, ctx->st));
     ctx->stats = PgxStats();
     CK(cudaEventRecord(ctx->ev[EV_PAIR0], ctx->st));
-    MRET(pgx::pair_streams_gpu(ctx->st, n_pairs, d_t, d_ti, d_c, d_ci, d_n, d_seed, d_slot, d_gi, d_m, d_frames,
+    MRET(pgx::pair_streams_gpu(ctx->st, n_pairs, d_t, d_ti, d_c, d_ci, d_n, d_seed, d_slot, d_at, d_m, d_frames,
                                ctx->mixed.err));
     std::vector<int> m(n_pairs);
     CK(cudaMemcpyAsync(m.data(), d_m, (size_t)n_pairs * 4, cudaMemcpyDeviceToHost, ctx->st));
@@ -612,7 +612,7 @@ int pgx_draw_pair_batch_gpu(PgxContext *ctx, int n_pairs, const PhTarget *t, con
     RET(ensure(ctx, ctx->x_draw_ps, (size_t)std::max(off, 1LL) * 12 * 8));
     double *d_out = P<double>(ctx->x_draw_ps);
     CK(cudaMemcpyAsync(d_off, clone_off, (size_t)(n_pairs + 1) * 4, cudaMemcpyHostToDevice, ctx->st));
-    MRET(pgx::draw_pairs_gpu(ctx->st, n_pairs, (int)off, d_t, d_ti, d_c, d_ci, d_seed, d_slot, d_off, d_gi, d_frames,
+    MRET(pgx::draw_pairs_gpu(ctx->st, n_pairs, (int)off, d_t, d_ti, d_c, d_ci, d_slot, d_off, d_at, d_frames,
                              d_out, ctx->mixed.err));
     CK(cudaEventRecord(ctx->ev[EV_PAIR1], ctx->st));
     if (off > 0) CK(cudaMemcpyAsync(ps, d_out, (size_t)off * 12 * 8, cudaMemcpyDeviceToHost, ctx->st));

@@ -168,4 +168,10 @@ PGX_HD float fast_rsqrt(float x) {
 #endif
 }
 
+// ---- the random streams -------------------------------------------------------------------------------------------
+// splitmix64: the state grows by kGolden at each output, so a place in a stream is a state, and the state after n Gaussians
+// (two outputs each) follows from any other modulo 2^64, with no count that could overflow
+constexpr uint64_t kGolden = 0x9E3779B97F4A7C15ULL;
+PGX_HD uint64_t after_gaussians(uint64_t state, uint64_t n) { return state + 2 * n * kGolden; }
+
 }  // namespace pgx

@@ -225,14 +225,14 @@ __device__ double safe_u(double value, double e) {
     return r > 9.5 ? 0.0 : (r > 0 ? exp(-0.5 * r * r) * (1.0 + 1e-9) : 2.0);
 }
 
-// Where the clones of pair q begin in its stream: gi[slot[q] + k] = the Gaussians taken before its k-th successful clone,
+// Where the clones of pair q begin in its stream: at[slot[q] + k] = the state before its k-th successful clone,
 // m[q] = how many succeed of n_clones[q] (as ph_pair_draw takes them: a target or a cluster that fails all its tries
 // drops the clone).  Lane l of a warp looks at the clone l after the next one as if none before it drew again; the
 // clones before the first that does are settled together, that one is walked through, and the rest look again.
 __global__ void k_pair_streams(int n_pairs, const PhTarget *__restrict__ t, const int *__restrict__ ti,
                                const PhCluster *__restrict__ c, const int *__restrict__ ci,
                                const int *__restrict__ n_clones, const uint64_t *__restrict__ seed,
-                               const long long *__restrict__ slot, int *__restrict__ gi, int *__restrict__ m,
+                               const long long *__restrict__ slot, uint64_t *__restrict__ at, int *__restrict__ m,
                                PairFrames *__restrict__ frames) {
     const unsigned all = 0xffffffffu;
     const int q = (int)(((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
@@ -244,39 +244,35 @@ __global__ void k_pair_streams(int n_pairs, const PhTarget *__restrict__ t, cons
     const double ut = tq.plx > 0 ? safe_u(tq.plx, tq.e_plx)
                                  : (tq.dist_pc > 1e-100 && tq.dist_pc < 1e100 && fabs(tq.e_lndist) < 10.0 ? 0.0 : 2.0);
     const double uc = safe_u(cq.dist_pc, cq.e_dist_pc);
-    const uint64_t s = seed[q];
-    int *o = gi + slot[q];
+    uint64_t *o = at + slot[q];
     const int n = n_clones[q];
-    int g0 = 0, k = 0;                                            // Gaussians taken, clones that succeeded
-    auto uniform = [&](int g) {                                   // the first deviate of Gaussian g
-        return (double)(splitmix_mix(s + (2 * (uint64_t)g + 1) * kGolden) >> 11) * (1.0 / 9007199254740992.0);
-    };
-    auto gauss = [&](int g) {
-        Rng r{s + 2 * (uint64_t)g * kGolden};
-        return r.gauss();
-    };
+    uint64_t s = seed[q];                                         // the stream's state before clone j
+    int k = 0;                                                    // clones that succeeded
+    auto uniform = [](uint64_t g) { return Rng{g}.uniform(); };   // the first deviate of the Gaussian at g
+    auto gauss = [](uint64_t g) { return Rng{g}.gauss(); };
     for (int j = 0; j < n;) {
-        const int g = g0 + 8 * lane;
+        const uint64_t g = after_gaussians(s, 8 * lane);
         bool bad = false;
         if (j + lane < n) {
+            const uint64_t gc = after_gaussians(g, 4);
             if (uniform(g) < ut) bad = !(target_plx(tq, gauss(g)) > 0);
-            if (uniform(g + 4) < uc) bad = bad || !(cluster_dist(cq, gauss(g + 4)) > 0);
+            if (uniform(gc) < uc) bad = bad || !(cluster_dist(cq, gauss(gc)) > 0);
         }
         const unsigned again = __ballot_sync(all, bad);
         const int good = min(again ? __ffs(again) - 1 : 32, n - j);
         if (lane < good) o[k + lane] = g;
         k += good;
         j += good;
-        g0 += 8 * good;
+        s = after_gaussians(s, 8 * good);
         if (again && j < n) {                                     // clone j, try by try (every lane alike)
-            const int start = g0;
+            const uint64_t start = s;
             int a = 0, b = 0;
-            while (a < kTries && !(target_plx(tq, gauss(g0)) > 0)) { a++; g0++; }
+            while (a < kTries && !(target_plx(tq, gauss(s)) > 0)) { a++; s = after_gaussians(s, 1); }
             if (a < kTries) {
-                g0 += 4;
-                while (b < kTries && !(cluster_dist(cq, gauss(g0)) > 0)) { b++; g0++; }
+                s = after_gaussians(s, 4);
+                while (b < kTries && !(cluster_dist(cq, gauss(s)) > 0)) { b++; s = after_gaussians(s, 1); }
                 if (b < kTries) {
-                    g0 += 4;
+                    s = after_gaussians(s, 4);
                     if (lane == 0) o[k] = start;
                     k++;
                 }
@@ -291,9 +287,9 @@ __global__ void k_pair_streams(int n_pairs, const PhTarget *__restrict__ t, cons
 // the FP64 pipe (eight Gaussians: log, cos and sqrt each); the pair is found by bisection, the frames come precomputed.
 __global__ void __launch_bounds__(128) k_draw_pairs(int n_pairs, int n, const PhTarget *__restrict__ t,
                                                     const int *__restrict__ ti, const PhCluster *__restrict__ c,
-                                                    const int *__restrict__ ci, const uint64_t *__restrict__ seed,
-                                                    const long long *__restrict__ slot, const int *__restrict__ off,
-                                                    const int *__restrict__ gi, const PairFrames *__restrict__ frames,
+                                                    const int *__restrict__ ci, const long long *__restrict__ slot,
+                                                    const int *__restrict__ off, const uint64_t *__restrict__ at,
+                                                    const PairFrames *__restrict__ frames,
                                                     double *__restrict__ ps) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -302,7 +298,7 @@ __global__ void __launch_bounds__(128) k_draw_pairs(int n_pairs, int n, const Ph
         const int mid = (q + hi) >> 1;
         if (off[mid] <= i) q = mid; else hi = mid;
     }
-    Rng g{seed[q] + 2 * (uint64_t)gi[slot[q] + (i - off[q])] * kGolden};
+    Rng g{at[slot[q] + (i - off[q])]};
     double *o = ps + 12 * (size_t)i;
     sample_target(t[ti[q]], frames[q].f[0], &g, o);
     sample_cluster(c[ci[q]], frames[q].f[1], &g, o + 6);
@@ -325,19 +321,19 @@ int draw_clusters_gpu(cudaStream_t st, int n, const PhCluster *c, int n_samp, co
 size_t pair_frames_bytes(int n_pairs) { return (size_t)n_pairs * sizeof(PairFrames); }
 
 int pair_streams_gpu(cudaStream_t st, int n_pairs, const PhTarget *t, const int *ti, const PhCluster *c, const int *ci,
-                     const int *n_clones, const uint64_t *seed, const long long *slot, int *gi, int *m, void *frames,
+                     const int *n_clones, const uint64_t *seed, const long long *slot, uint64_t *at, int *m, void *frames,
                      std::string &err) {
     k_pair_streams<<<(unsigned)(((size_t)n_pairs * 32 + 127) / 128), 128, 0, st>>>(
-        n_pairs, t, ti, c, ci, n_clones, seed, slot, gi, m, static_cast<PairFrames *>(frames));
+        n_pairs, t, ti, c, ci, n_clones, seed, slot, at, m, static_cast<PairFrames *>(frames));
     return check(cudaGetLastError(), err, "k_pair_streams");
 }
 
 int draw_pairs_gpu(cudaStream_t st, int n_pairs, int n, const PhTarget *t, const int *ti, const PhCluster *c,
-                   const int *ci, const uint64_t *seed, const long long *slot, const int *off, const int *gi,
-                   const void *frames, double *ps, std::string &err) {
+                   const int *ci, const long long *slot, const int *off, const uint64_t *at, const void *frames,
+                   double *ps, std::string &err) {
     if (n <= 0) return 0;
     k_draw_pairs<<<(unsigned)(((size_t)n + 127) / 128), 128, 0, st>>>(
-        n_pairs, n, t, ti, c, ci, seed, slot, off, gi, static_cast<const PairFrames *>(frames), ps);
+        n_pairs, n, t, ti, c, ci, slot, off, at, static_cast<const PairFrames *>(frames), ps);
     return check(cudaGetLastError(), err, "k_draw_pairs");
 }
 

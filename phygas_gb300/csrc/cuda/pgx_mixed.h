@@ -40,19 +40,19 @@ int block_tables(cudaStream_t st, int N, int nmax, const int *npts, const double
                  const double *R2, float4 *blk, std::string &err);
 // the draws from the measurement errors on the device (pgx_draws.cu): targets' and clusters' nominal states and
 // covariances (seed[i] = ph_seed("lin", id)), and the clones of pairs (seed[q] = ph_seed(id, name)) in two steps: where
-// each clone begins in its pair's stream (gi at slots slot[q], successful clones m[q], the pairs' frames), then the n
-// successful clones at off[q]; every pointer is device memory
+// each clone begins in its pair's stream (the states `at` at slots slot[q], successful clones m[q], the pairs' frames),
+// then the n successful clones at off[q]; every pointer is device memory
 int draw_targets_gpu(cudaStream_t st, int n, const PhTarget *t, int n_samp, const uint64_t *seed, double *ps0,
                      double *sig, std::string &err);
 int draw_clusters_gpu(cudaStream_t st, int n, const PhCluster *c, int n_samp, const uint64_t *seed, double *ps0,
                       double *sig, std::string &err);
 size_t pair_frames_bytes(int n_pairs);
 int pair_streams_gpu(cudaStream_t st, int n_pairs, const PhTarget *t, const int *ti, const PhCluster *c, const int *ci,
-                     const int *n_clones, const uint64_t *seed, const long long *slot, int *gi, int *m, void *frames,
+                     const int *n_clones, const uint64_t *seed, const long long *slot, uint64_t *at, int *m, void *frames,
                      std::string &err);
 int draw_pairs_gpu(cudaStream_t st, int n_pairs, int n, const PhTarget *t, const int *ti, const PhCluster *c,
-                   const int *ci, const uint64_t *seed, const long long *slot, const int *off, const int *gi,
-                   const void *frames, double *ps, std::string &err);
+                   const int *ci, const long long *slot, const int *off, const uint64_t *at, const void *frames,
+                   double *ps, std::string &err);
 // the cluster table cluster-major (blk [nblk][nc][4] -> [nc][nblk][4], c32 [ncp][nc][3] -> [nc][ncp][3], lm
 // [ncp][nc] -> [nc][lm_pitch]): the staged filter's bulk copies read contiguous ranges
 int cluster_major(cudaStream_t st, int nc, int ncp, int nblk, int lm_pitch, const float4 *blk, const float4 *c32,
