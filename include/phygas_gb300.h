@@ -191,11 +191,12 @@ int pgx_pair(PgxContext *ctx, int n_pairs, const int *clone_off, const double *p
 
 /* Launch-shape autotuner of the clone kernel (no counterpart in the reference): runs the batch (the arguments of
  * pgx_pair) with every shape this build has -- warps per block x clones traced per lane x resident blocks per SM
- * asked of the compiler (a register cap) -- and keeps the fastest for
- * this context's later pgx_pair calls.  ms[pgx_pair_shapes()] (or NULL) gets each shape's device time; *best (or NULL)
- * its index.  Every shape must give the same bits: a shape whose results differ fails the call (PGX_E_CUDA).
- * Batches whose pairs all have at most 1024 clones run as one captured CUDA graph (prep, persistent trace, reduce)
- * replayed with the batch's parameters; the tuner's runs also capture each shape's graph. */
+ * asked of the compiler (a register cap) -- and keeps the fastest for this context's later batches of more than 32
+ * clones per SM; smaller ones always take a kernel of their own, eight lanes per clone, which is not one of the shapes.
+ * ms[pgx_pair_shapes()] (or NULL) gets each shape's device time; *best (or NULL) its index.  Every shape, and the
+ * small batches' kernel, must give the same bits: one whose results differ fails the call (PGX_E_CUDA).
+ * Every batch runs as a captured CUDA graph (prep, persistent trace, reduce) replayed with the batch's parameters; the
+ * tuner's runs also capture each shape's graph.  Pairs of more than 1024 clones are reduced after it. */
 int pgx_tune_pair(PgxContext *ctx, int n_pairs, const int *clone_off, const double *ps, const int *steps,
                   const double *dt, const double *r50_pc, const double *rtot_pc, double *ms, int *best);
 /* Launch-shape autotuner of the screen's block filter (no counterpart in the reference): screens the staged chunk

@@ -528,7 +528,8 @@ class Context:
         return (res, clones) if want_clones else res
 
     def tune_pair(self, clone_off, ps, steps, dt, r50_pc, rtot_pc):
-        """Time every launch shape of the clone kernel on this batch and keep the fastest (pgx_tune_pair):
+        """Time every launch shape of the clone kernel on this batch and keep the fastest for batches of more than 32
+        clones per SM (pgx_tune_pair):
         -> (index of the chosen shape, [(warps per block, clones per lane, min blocks per SM, ms), ...])."""
         args = [np.ascontiguousarray(clone_off, np.int32), np.ascontiguousarray(ps, np.float64),
                 np.ascontiguousarray(steps, np.int32), np.ascontiguousarray(dt, np.float64),

@@ -1646,14 +1646,16 @@ int pgx_tune_pair(PgxContext *ctx, int n_pairs, const int *clone_off, const doub
     std::vector<PhResult> ref(n_pairs), got(n_pairs);
     int b = 0;
     double bms = 0;
+    // the small batches' kernel first, for its results alone: it takes them whatever the tuner finds
+    RET(pair_run(ctx, pgx::mc_quad_variant(), n_pairs, clone_off, ps, steps, dt, r50_pc, rtot_pc, ref.data(), nullptr));
     for (int v = 0; v < nv; v++) {
-        PhResult *out = v == 0 ? ref.data() : got.data();
+        PhResult *out = got.data();
         // twice: the first run of a shape also captures and instantiates its graph
         RET(pair_run(ctx, v, n_pairs, clone_off, ps, steps, dt, r50_pc, rtot_pc, out, nullptr));
         RET(pair_run(ctx, v, n_pairs, clone_off, ps, steps, dt, r50_pc, rtot_pc, out, nullptr));
         const double t = ctx->stats.ms_pair;
         if (ms) ms[v] = t;
-        if (v > 0 && memcmp(ref.data(), got.data(), sizeof(PhResult) * (size_t)n_pairs) != 0)
+        if (memcmp(ref.data(), got.data(), sizeof(PhResult) * (size_t)n_pairs) != 0)
             return fail(ctx, PGX_E_CUDA, "pgx_tune_pair: launch shape %d changed the results", v);
         if (v == 0 || t < bms) { b = v; bms = t; }
     }
