@@ -141,13 +141,14 @@ PGX_HD double rcp_refine(double d, double y) {
 
 // Reciprocal and reciprocal square root on the GPU's fast units: within 2 ulp (4 eps relative) by their documented
 // worst case (PTX rcp.approx.f32: 1 ulp; rsqrt.approx.f32: relative error 2^-22.9; both over the full range).  The
-// .ftz forms flush subnormal arguments and results, which never occur here: every argument is checked or clamped to
-// be at least 1e-30, and a reciprocal's argument at most 1e30, so arguments and results are normal -- and they issue
-// as one special-function instruction, without the subnormal scaling around it.  Host builds use the exact operations,
-// which the same margins cover, scaled by (1 + host_fast_err): a host test sets it to put the results at either end
-// of the device units' error band (it is 0 otherwise, and does not exist in device code).
+// .ftz forms take a subnormal argument as zero and flush a subnormal result -- a reciprocal above 2^126 is 0 -- and issue
+// as one special-function instruction, without the subnormal scaling around it.  Callers check or clamp their arguments to
+// be at least 1e-30; where one can pass 2^126, what the zero does to the result is said there.  Host builds use the exact
+// operations with the same flushing, which the same margins cover, scaled by (1 + host_fast_err): a host test sets it to
+// put the results at either end of the device units' error band (it is 0 otherwise, and does not exist in device code).
 #ifndef __CUDA_ARCH__
 inline float host_fast_err = 0.f;
+inline float host_ftz(float x) { return fabsf(x) < 0x1p-126f ? copysignf(0.f, x) : x; }
 #endif
 PGX_HD float fast_rcp(float x) {
 #ifdef __CUDA_ARCH__
@@ -155,7 +156,7 @@ PGX_HD float fast_rcp(float x) {
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 #else
-    return 1.f / x * (1.f + host_fast_err);
+    return host_ftz(1.f / host_ftz(x) * (1.f + host_fast_err));
 #endif
 }
 PGX_HD float fast_rsqrt(float x) {
@@ -164,7 +165,7 @@ PGX_HD float fast_rsqrt(float x) {
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 #else
-    return 1.f / sqrtf(x) * (1.f + host_fast_err);
+    return host_ftz(1.f / sqrtf(host_ftz(x)) * (1.f + host_fast_err));
 #endif
 }
 

@@ -38,7 +38,9 @@ PGX_HD float ldl_form(float l10, float l20, float l21, float i1, float i2, float
 // f(t) = q_m + 2 b t + q_d t^2 at the clamped -b / q_d.  The factors are those of one M' near M, so f loses the factor
 // 1 - rho once; each solve's own error (4 eps tr(M) / lam relative to M', 5.7 with second-order terms), the rounding of d
 // (an eps of each component: eps sqrt(tr / lam) in the norm) and of the forms and the polynomial enter against (sqrt(q_m) +
-// T sqrt(q_d))^2 <= 2 (q_m + T^2 q_d): rho is 24 eps tr / lam, so 0.7 rho + 40 eps of that sum covers them.  About five
+// T sqrt(q_d))^2 <= 2 (q_m + T^2 q_d): rho is 24 eps tr / lam, so 0.7 rho + 40 eps of that sum covers them.  Above 2^126 the
+// reciprocal of q_d is flushed and t is not the minimum: the sum is formed at a scale (T^2 >= 4) where it is infinite then,
+// and the bound not a number or minus infinity, which settles nothing.  About five
 // instructions more than the triangle inequality |m| - T |d|, which settled 71.1 % of the blocks of 2,000 stars x 4,087
 // clusters where this settles 73.8 %, and left 19.4 % of the walked points where this leaves 17.4 % (filter 3.43 -> 3.25 ms).
 PGX_HD float ldl_line_min(float l10, float l20, float l21, float i1, float i2, float i3, const float (&m)[3],
@@ -50,7 +52,8 @@ PGX_HD float ldl_line_min(float l10, float l20, float l21, float i1, float i2, f
     const float qd = fmaf(d2 * d2, i3, fmaf(d1 * d1, i2, dx * dx * i1));
     const float t = fminf(fmaxf(-b * fast_rcp(fmaxf(qd, 1e-30f)), lo), hi);
     const float f = fmaf(t, fmaf(t, qd, 2.f * b), qm);
-    return fmaf(-fmaf(0.7f, rho, 40.f * kEps32), fmaf(T2, qd, qm), f) * (1.f - rho);
+    const float up = T2 < 4.f ? 4.f : 1.f;
+    return fmaf(-fmaf(0.7f / up, rho, 40.f / up * kEps32), fmaf(up * T2, qd, up * qm), f) * (1.f - rho);
 }
 
 // The reference's trace bound (chi2 >= dist^2 / trace M over the step's segment) with FP32 margins: the exact
@@ -145,8 +148,8 @@ constexpr float kBlkTau = PGX_BLK_TAU;        // Myr: the largest |tau| in a blo
 
 // The point test against a block's dominating matrix N = S_t + S_c (the block tables of the point's block) in place of
 // the point's own M(k): M(k) <= N, so every form in M(k)^-1 is at least the form in N^-1; lam <= lambda_min(N), and
-// the FP64 adjugate's rounding at M(k) from tr(N) / lam_lo as in the block test.  Otherwise point_skip32's triangle
-// test on the step's segment.
+// the FP64 adjugate's rounding at M(k) from tr(N) / lam_lo as in the block test.  Otherwise the triangle inequality on the
+// step's segment, |m0| - |dr|.
 PGX_HD bool point_skip32_blk(const float4 (&bt)[4], const float4 (&bc)[4], const float (&m0)[3], const float (&m1)[3],
                              float cut) {
     const float N0 = bt[2].x + bc[2].x, N1 = bt[2].y + bc[2].y, N2 = bt[2].z + bc[2].z;
@@ -268,14 +271,19 @@ PGX_HD bool point_bound32(const float (&St)[6], const float (&Sc)[6], float lmt,
     const float dd = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
     const float m00 = fmaf(m0[0], m0[0], fmaf(m0[1], m0[1], m0[2] * m0[2]));
     const float m11 = fmaf(m1[0], m1[0], fmaf(m1[1], m1[1], m1[2] * m1[2]));
-    if (trace_far32(a, dd, m00, m11, tr, lam, cut)) return false;
+    const float mm = fmaxf(m00, m11);
+    const bool wild = !(tr < 1e10f && mm < 1e18f);
+    if (!wild && trace_far32(a, dd, m00, m11, tr, lam, cut)) return false;
     constexpr float up = 1.f + 8.f * kEps32, down = 1.f - 8.f * kEps32;
-    if (!(lam > 1e-30f)) {
+    // Within wild's limits (a spread of 10^5 kpc, a separation of 10^9) no product below overflows and no reciprocal of a
+    // quantity that a bound shrinks with is flushed; det and c2 stay below 1e30, and where the cube of 1 + rho does not,
+    // its reciprocal's zero makes det_lo zero.
+    if (wild || !(lam > 1e-30f)) {
         b.lb = 0.f;
         b.ub = inf;
         return true;
     }
-    const float big = fast_sqrt(fmaxf(m00, m11)) * up;
+    const float big = fast_sqrt(mm) * up;
     const float n0 = fast_sqrt(m00) * up;
     const float dr_err = 8.f * kEps32 * big + 1e-12f;   // |FP32 dr - FP64 dr|: the rounding of m0 and m1
     float s = 0.f;
