@@ -181,11 +181,11 @@ int pgx_tracks(PgxContext *ctx, int n, const double *ps, const int *npts, double
  * r50_pc/rtot_pc per pair.  res[n_pairs] gets the results; clone_out (NULL or 3 x total: best kpc, tbest Myr,
  * vbest kpc/Myr, clone-major blocks) the per-clone closest approaches.
  * What the orbits run on, here and in every other call that traces clones: positions and displacements of a step are
- * 64-bit integers (2^-55 and 2^-61 kpc and finer) and the force is evaluated on pairs of floats (2^-47 relative), in FP64
- * within 14 |dt| kpc of the centre (dt in Myr), for 0.01 <= |dt| <= 0.125 Myr, starts outside 0.4 and 14 |dt| kpc and
- * orbits within 2,048 kpc; everything else is traced in FP64.  Over that range the orbits end no further from exact
- * arithmetic than FP64 steps do (5 to 20 times nearer on galactic orbits); the two differ by FP64's rounding, some 1e-13
- * of the results. */
+ * 64-bit integers (2^-55 and 2^-61 kpc, finer on short steps and small orbits; positions coarser beyond 256 kpc) and the
+ * force is evaluated on pairs of floats (2^-47 relative), within 12 |dt| kpc of the centre (dt in Myr; at least 0.4) its
+ * dominant part, the bulge's, in FP64, for 0.01 <= |dt| <= 0.125 Myr, starts 0.15 kpc and more from the centre and orbits within 10^6 kpc; everything
+ * else is traced in FP64.  Over that range the orbits end no further from exact arithmetic than FP64 steps do (5 to 50
+ * times nearer on galactic orbits); the two differ by FP64's rounding, some 1e-13 of the results. */
 int pgx_pair(PgxContext *ctx, int n_pairs, const int *clone_off, const double *ps, const int *steps,
              const double *dt, const double *r50_pc, const double *rtot_pc, PhResult *res, double *clone_out);
 

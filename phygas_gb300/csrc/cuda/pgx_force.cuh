@@ -143,16 +143,20 @@ __device__ __noinline__ Accel mw_accel_any(double x, double y, double z) {
     return a;
 }
 
-// the force of the FP32 orbit's steps near the centre (orbit32_accel), out of line: a few steps of few orbits
-struct MwForce64 {
-    __device__ __forceinline__ void operator()(double x, double y, double z, double *a) const { mw_accel(x, y, z, a[0], a[1], a[2]); }
+// the FP32 orbit's force near the centre (accel_near), out of line: some steps of few orbits
+struct MwBulge64 {
+    __device__ __forceinline__ double operator()(double r2) const {
+        const double i = rsqrt_h3(r2 + kBulgeB2);
+        return (i * i) * (i * -kBulgeGM);
+    }
 };
-__device__ __noinline__ Acc64i mw_accel_near(const OrbitScale s, double dt, int64_t x, int64_t y, int64_t z) {
-    return accel_near(MwForce64(), s, dt, x, y, z);
+__device__ __noinline__ Acc64i mw_accel_near(const Force32 K, const OrbitScale s, double dt, int64_t x, int64_t y, int64_t z) {
+    return accel_near<MwModel32>(K, HaloTable32(), MwBulge64(), s, dt, x, y, z);
 }
 struct MwNear {
-    __device__ __forceinline__ Acc64i operator()(const OrbitScale &s, double dt, int64_t x, int64_t y, int64_t z) const {
-        return mw_accel_near(s, dt, x, y, z);
+    __device__ __forceinline__ Acc64i operator()(const Force32 &K, const OrbitScale &s, double dt, int64_t x, int64_t y,
+                                                 int64_t z) const {
+        return mw_accel_near(K, s, dt, x, y, z);
     }
 };
 
@@ -287,9 +291,15 @@ __device__ __forceinline__ int64_t quad_accel32(const F3 &k, float c, int64_t x,
     const F2 g1 = f2_add(quad_shfl(e, 2), quad_shfl(e, 0)), fd = quad_shfl(e, 1), fz = quad_shfl(ez, 1);
     return acc_to_fixed(f2_mul(f2_norm(f2_add(g1, f2_pick(role == 2, fz, fd))), f));
 }
-// the lane's coordinate of mw_accel_near: quad_accel's bits are mw_accel's (every lane of the warp calls)
-__device__ __noinline__ int64_t quad_accel_near(const OrbitScale s, double dt, int64_t x, int role) {
-    return f64_to_i64(quad_accel((double)x * pow2(s.e - 55), role) * (dt * dt * pow2(61 - s.e + s.k)));
+// mw_accel_near's coordinate of the lane, its operations on four lanes (every lane of the warp calls)
+__device__ __noinline__ int64_t quad_accel_near(const F3 k, const OrbitScale s, double dt, int64_t x, int role) {
+    const unsigned all = 0xffffffffu;
+    float r2;
+    const int64_t a = quad_accel32(role == 0 ? F3{0.f, 0.f, 0.f} : k, s.c, x, role, r2);
+    const double q = (double)x * pow2(s.e - 55);
+    const double X = __shfl_sync(all, q, 0, 4), Y = __shfl_sync(all, q, 1, 4), Z = __shfl_sync(all, q, 2, 4);
+    const double g = MwBulge64()(fma(X, X, fma(Y, Y, Z * Z))) * (dt * dt * pow2(61 - s.e + s.k));
+    return a + f64_to_i64(g * q);
 }
 
 }  // namespace pgx

@@ -466,12 +466,12 @@ __device__ __forceinline__ bool in_range32(float ra, float rb, float rmax) {
 }
 
 // the scale of a clone's two orbits (false: none, NaN and infinities included)
-__device__ __forceinline__ bool clone_scale(const double *p, int steps, double dt, float near2, OrbitScale &s) {
+__device__ __forceinline__ bool clone_scale(const double *p, int steps, double dt, OrbitScale &s) {
     double va, vb, sum = 0.0;
     const double ra = orbit32_reach(p, p + 3, steps, dt, va), rb = orbit32_reach(p + 6, p + 9, steps, dt, vb);
 #pragma unroll
     for (int j = 0; j < 12; j++) sum += p[j];                 // fmax passes over NaN
-    return fabs(sum) < 1e300 && orbit32_start_ok(p, near2) && orbit32_start_ok(p + 6, near2) &&
+    return fabs(sum) < 1e300 && orbit32_start_ok(p) && orbit32_start_ok(p + 6) &&
            orbit32_units(fmax(ra, rb), fmax(va, vb), dt, s);
 }
 
@@ -489,8 +489,8 @@ struct SlowStep {
 };
 // false: an orbit too close to the centre
 __device__ __noinline__ bool slow_step(SlowStep &t, int i, double dt) {
-    if (t.ra < t.near2) t.A = mw_accel_near(t.s, dt, t.a.x, t.a.y, t.a.z);            // (as orbit32_accel)
-    if (t.rb < t.near2) t.B = mw_accel_near(t.s, dt, t.b.x, t.b.y, t.b.z);
+    if (t.ra < t.near2) t.A = mw_accel_near(t.K, t.s, dt, t.a.x, t.a.y, t.a.z);            // (as orbit32_accel)
+    if (t.rb < t.near2) t.B = mw_accel_near(t.K, t.s, dt, t.b.x, t.b.y, t.b.z);
     if (!(fminf(t.ra, t.rb) > kOrbit32MinR2)) return false;
     if (t.done) return true;
     t.n.step(t.dd, t.q1, t.b1, t.s,
@@ -525,7 +525,7 @@ struct Clone32 {
         n.pend = false;
         n.tie = 0;
         near2 = orbit32_near2(dt);
-        ok = clone_scale(p, steps, dt, near2, s);
+        ok = clone_scale(p, steps, dt, s);
         if (!ok) {                                            // (stepped along where its lane has another clone)
             a = b = Orbit32{};
             K = Force32{};
@@ -536,8 +536,11 @@ struct Clone32 {
         K = force32_constants<MwModel32>(dt, s);
         rmax = orbit32_max_r2(s);
         float ra, rb;
-        orbit32_start<MwModel32>(a, K, HaloTable32(), s, p, p + 3, dt, ra);
-        orbit32_start<MwModel32>(b, K, HaloTable32(), s, p + 6, p + 9, dt, rb);
+        auto accel = [&](long long x, long long y, long long z, float &r2) {
+            return mw_accel32(K, s, dt, near2, x, y, z, r2);
+        };
+        orbit32_start(a, accel, s, p, p + 3, dt, ra);
+        orbit32_start(b, accel, s, p + 6, p + 9, dt, rb);
         ok = in_range32(ra, rb, rmax);
         n.start(p, s);
         return true;
@@ -576,6 +579,17 @@ struct Clone32 {
     __device__ __forceinline__ int fp64_steps(int steps) const { return ok ? min(n.tie, steps) : max(steps, 1); }
 };
 
+// orbit32_accel on four lanes (every lane of the warp calls)
+__device__ __forceinline__ long long quad_step_accel(const F3 &k, const OrbitScale &s, double dt, float near2, long long x,
+                                                     int role, float &r2) {
+    long long a = quad_accel32(k, s.c, x, role, r2);
+    if (__any_sync(0xffffffffu, r2 < near2)) {
+        const long long f = quad_accel_near(k, s, dt, x, role);
+        if (r2 < near2) a = f;
+    }
+    return a;
+}
+
 // The same clone on eight lanes (quad_accel32: target on lanes 0-3 of the eight, cluster on 4-7): the same bits.
 struct QuadClone32 {
     long long x, w;          // the lane's coordinate and displacement
@@ -605,7 +619,7 @@ struct QuadClone32 {
 #pragma unroll
         for (int j = 0; j < 12; j++) p[j] = ps[j];
         near2 = orbit32_near2(dt);
-        ok = clone_scale(p, steps, dt, near2, s);
+        ok = clone_scale(p, steps, dt, s);
         if (!ok) {                                            // (traced along with its warp, and again in FP64)
             s = OrbitScale{0x1p-23f, 0};
             near2 = 0.f;
@@ -617,8 +631,8 @@ struct QuadClone32 {
         const double v = role == 0 ? ps[o + 3] : (role == 1 ? ps[o + 4] : ps[o + 5]);
         x = ok && role < 3 ? f64_to_i64(q * pow2(55 - s.e)) : 0;
         float r2;
-        const long long a = quad_accel32(k, s.c, x, role, r2);
-        w = (ok && role < 3 ? displacement(v, dt, pow2(61 - s.e + s.k)) + a / 2 : 0) + (32LL << s.k);
+        const long long a = quad_step_accel(k, s, dt, near2, x, role, r2);
+        w = (ok && role < 3 ? displacement(v, dt, pow2(61 - s.e + s.k)) + a / 2 : 0) + (1LL << (5 + s.k));
         const float rb = __shfl_xor_sync(0xffffffffu, r2, 4);        // (every lane, whatever its ok)
         ok = ok && in_range32(r2, rb, rmax);
         n.start(p, s);
@@ -639,7 +653,7 @@ struct QuadClone32 {
         const bool near = fminf(r2, rb) < near2, done = n.quick(dd, q1, b1);
         if (__any_sync(all, ok && (near || !done))) {
             if (__any_sync(all, ok && near)) {                        // (as orbit32_accel)
-                const long long m = quad_accel_near(s, dt, x, role);
+                const long long m = quad_accel_near(k, s, dt, x, role);
                 if (ok && r2 < near2) a = m;
                 ok = ok && fminf(r2, rb) > kOrbit32MinR2;
             }
@@ -679,7 +693,7 @@ static __global__ void __launch_bounds__(32) k_coarse_tracks(int N, const double
     for (int j = 0; j < 6; j++) p12[j] = p12[6 + j] = q[j];
     OrbitScale s;
     float near2 = orbit32_near2(dt);
-    bool ok = clone_scale(p12, (n - 1) * kSub, dt, near2, s);
+    bool ok = clone_scale(p12, (n - 1) * kSub, dt, s);
     if (!ok) {
         s = OrbitScale{0x1p-23f, 0};
         near2 = 0.f;
@@ -689,20 +703,15 @@ static __global__ void __launch_bounds__(32) k_coarse_tracks(int N, const double
     const double unit = unit64(s);
     long long x = ok && role < 3 ? f64_to_i64(q[c] * pow2(55 - s.e)) : 0;
     float r2;
-    const long long a0 = quad_accel32(k, s.c, x, role, r2);
+    const long long a0 = quad_step_accel(k, s, dt, near2, x, role, r2);
     ok = ok && in_range32(r2, r2, rmax);
-    long long w = (ok && role < 3 ? displacement(q[3 + c], dt, pow2(61 - s.e + s.k)) + a0 / 2 : 0) + (32LL << s.k);
+    long long w = (ok && role < 3 ? displacement(q[3 + c], dt, pow2(61 - s.e + s.k)) + a0 / 2 : 0) + (1LL << (5 + s.k));
     for (int j = 0; j < nw; j++) {
         if (j > 0) {
 #pragma unroll 1
             for (int m = 0; m < kSub; m++) {
                 x += orbit32_drift(w, 6 + s.k);
-                long long a = quad_accel32(k, s.c, x, role, r2);
-                if (__any_sync(all, r2 < near2)) {                    // (as orbit32_accel)
-                    const long long f = quad_accel_near(s, dt, x, role);
-                    if (r2 < near2) a = f;
-                }
-                w += a;
+                w += quad_step_accel(k, s, dt, near2, x, role, r2);
                 ok = ok && (j >= n || in_range32(r2, r2, rmax));
             }
         }

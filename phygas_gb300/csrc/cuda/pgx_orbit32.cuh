@@ -9,18 +9,20 @@
 //    between drifts added up), exact but for the last unit, which is 64 times finer than FP64's at 8 kpc;
 //  * the force is evaluated on pairs of floats (value = h + l, about 48 bits), each product and sum with its rounding
 //    error carried along by fused multiply-adds; the constants are the FP64 ones, in three floats.
-// The force's error, 2^-47.8 relative (rms) and random, enters w through a dt^2 ~ 2^-11 w, below FP64's own rounding
+// The force's error, 2^-47.2 relative (rms) and random, enters w through a dt^2 ~ 2^-11 w, below FP64's own rounding
 // of the velocity -- where an orbit turns slowly.  Within kOrbit32Near |dt| of the centre a dt is so large a part of v that
-// it is not: there the force is FP64's (orbit32_accel).
+// it is not: there the bulge's part, nearly all of it, is FP64's (accel_near; FP64 throughout is no nearer).
 //
 // What is traced this way is what comes out no further from exact arithmetic than FP64 steps, measured against 113-bit
-// arithmetic (tests/test_orbit32_range.py): 0.01 <= |dt| <= 0.125 Myr, a start outside kOrbit32Near |dt| and 0.4 kpc, and a reach of
-// less than 2,048 kpc.  2,000 steps of 0.05 Myr at 8 kpc: 1.3e-14 kpc rms, the FP64 step 8e-14; at 1 kpc 2e-14 and 7e-14;
-// at 1,024 kpc 1.6e-13 and 1.7e-12.  Beyond, and with less than 2^-10 kpc to the centre, a caller traces in FP64.
+// arithmetic (tests/test_orbit32_range.py): 0.01 <= |dt| <= 0.125 Myr, a start at least 0.15 kpc from the centre and a reach
+// of less than 10^6 kpc.  2,000 steps of 0.05 Myr end 8e-15 kpc off (rms; FP64 steps: 9e-14) at 8 kpc, 3e-14 (1.0e-13) at 1
+// kpc, 1e-14 (2.7e-12) at 1,000 kpc and 7e-13 (4.5e-11) at 100,000.  Other orbits, and those that come within 2^-10 kpc of
+// the centre, a caller traces in FP64.
 //
-// The units.  Orbits larger than 256 kpc take units 2^e times larger; steps of 1/16 Myr and less take displacements 2^k
-// times finer, which FP64's rounding of a slow orbit's velocity asks for (OrbitScale).  FP64 rounds a position at 2,048 kpc
-// to 2^-42 kpc, 2^10 times this unit there; at 30,000 kpc and steps of 0.01 Myr a displacement's unit was the larger error.
+// The units (OrbitScale): orbits that reach 256 kpc and more take positions' units 2^e times larger, those that stay within 64
+// four times smaller.  A displacement's unit does not follow: it is 2^-61 kpc and finer at shorter steps, since FP64's
+// rounding of a slow orbit's velocity is finer too (with a unit that grew with the scale, orbits beyond 5,000 kpc and
+// slow ones at steps of 0.02 Myr came out up to ten times further off than FP64's).
 #pragma once
 #include <cstdint>
 #include "pgx_bits.cuh"
@@ -143,12 +145,13 @@ struct OrbitScale {
     float c;
     int e, k = 0;
 };
-constexpr double kOrbit32MinDt = 0.01, kOrbit32MaxDt = 0.125, kOrbit32MaxReach = 2048.0;
-constexpr double kOrbit32Near = 14.0, kOrbit32MinStart = 0.4;      // kpc per Myr of step; kpc
+constexpr double kOrbit32MinDt = 0.01, kOrbit32MaxDt = 0.125, kOrbit32MaxReach = 1e6;
+constexpr double kOrbit32Near = 12.0, kOrbit32NearMin = 0.4;       // kpc per Myr of step; kpc
+constexpr double kOrbit32MinStart = 0.15;
 constexpr float kOrbit32MinR2 = 0x1p-20f;
 
 PGX_HD float orbit32_near2(double dt) {
-    const double r = kOrbit32Near * dt;
+    const double r = fmax(kOrbit32Near * fabs(dt), kOrbit32NearMin);
     return (float)(r * r);
 }
 
@@ -156,28 +159,29 @@ PGX_HD float orbit32_near2(double dt) {
 PGX_HD bool orbit32_scale(double reach, double dt, OrbitScale &s) {
     const double d = fabs(dt);
     if (!(reach < kOrbit32MaxReach && d >= kOrbit32MinDt && d <= kOrbit32MaxDt)) return false;
-    s.e = 0;
-    s.c = 0x1p-23f;
+    s.e = reach < 64.0 ? -2 : 0;
+    s.c = reach < 64.0 ? 0x1p-25f : 0x1p-23f;
     for (double lim = 256.0; lim <= reach; lim *= 2.0) { s.e++; s.c *= 2.f; }
     return true;
 }
-// The scale with the displacements' own unit: k = 2 for steps of 1/16 Myr and less, 3 from 1/32, 4 from 1/64, and e more, so
-// that a larger orbit's displacements stay as fine -- less where v dt would leave a quarter of the integer's range
+// The scale with the displacements' own unit: 2^-61 kpc at any e, and as much finer as a dt^2 of shorter steps leaves its
+// integer room (to 2^-68 at 0.01 Myr) -- less where v dt would leave a quarter of the integer's range
 PGX_HD bool orbit32_units(double reach, double vdt, double dt, OrbitScale &s) {
     if (!orbit32_scale(reach, dt, s)) return false;
-    const double d = fabs(dt);
-    s.k = s.e + (d <= 0.015625 ? 4 : (d <= 0.03125 ? 3 : (d <= 0.0625 ? 2 : 0)));
+    s.k = s.e;
+    for (double t = kOrbit32MaxDt / dt * (kOrbit32MaxDt / dt); t >= 2.0; t *= 0.5) s.k++;
     while (s.k > 0 && vdt >= pow2(s.e - s.k - 1)) s.k--;
     return vdt < pow2(s.e - s.k - 1);
 }
-// The reach to ask for an orbit from q, v over `steps` steps: twice the straight line's, but under 0.4 kpc/Myr within 20 kpc
-// an orbit is bound and stays inside 200 kpc (one that does not is noticed: orbit32_max_r2)
+// The reach to ask for an orbit from q, v over `steps` steps: twice the straight line's, but an orbit of 0.3 kpc/Myr within
+// 3 kpc hardly leaves 30 kpc and one of 0.4 within 20 kpc 200 (one that does is noticed: orbit32_max_r2)
 PGX_HD double orbit32_reach(const double *q, const double *v, double steps, double dt, double &vdt) {
     const double x = fmax(fabs(q[0]), fmax(fabs(q[1]), fabs(q[2])));
     const double u = fmax(fabs(v[0]), fmax(fabs(v[1]), fabs(v[2])));
     vdt = u * fabs(dt);
     double drift = 2.0 * vdt * steps;
     if (u < 0.4 && x < 20.0) drift = fmin(drift, 200.0);
+    if (u < 0.3 && x < 3.0) drift = fmin(drift, 30.0);
     return fmax(2.0 * x + drift + 20.0, 512.0 * vdt);
 }
 // r2 below this: inside the positions' range
@@ -283,20 +287,23 @@ PGX_HD Acc64i accel32(const Force32 &K, const Table &table, float c, int64_t x, 
     return Acc64i{acc_to_fixed(a.x), acc_to_fixed(a.y), acc_to_fixed(a.z)};
 }
 
-// The force of a step that ends near the centre in FP64: force(x, y, z, a) gives a in kpc/Myr^2 at a position in kpc
-template <class F>
-PGX_HD Acc64i accel_near(const F &force, const OrbitScale &s, double dt, int64_t x, int64_t y, int64_t z) {
-    const double u = pow2(s.e - 55), w = dt * dt * pow2(61 - s.e + s.k);
-    double a[3];
-    force((double)x * u, (double)y * u, (double)z * u, a);
-    return Acc64i{f64_to_i64(a[0] * w), f64_to_i64(a[1] * w), f64_to_i64(a[2] * w)};
+// The force near the centre, where the bulge is nearly all of it: its part in FP64 (bulge(r2) = -GM (r2 + b^2)^-3/2), the
+// disk's and the halo's, a few percent, on pairs of floats
+template <class M, class Table, class Bulge>
+PGX_HD Acc64i accel_near(const Force32 &K, const Table &table, const Bulge &bulge, const OrbitScale &s, double dt, int64_t x,
+                         int64_t y, int64_t z) {
+    float r2;
+    const Acc64i a = accel32<M>(Force32{F3{0.f, 0.f, 0.f}, K.disk, K.halo}, table, s.c, x, y, z, r2);
+    const double u = pow2(s.e - 55), X = (double)x * u, Y = (double)y * u, Z = (double)z * u;
+    const double g = bulge(fma(X, X, fma(Y, Y, Z * Z))) * (dt * dt * pow2(61 - s.e + s.k));
+    return Acc64i{a.x + f64_to_i64(g * X), a.y + f64_to_i64(g * Y), a.z + f64_to_i64(g * Z)};
 }
-// a step's force: on pairs of floats, within near2 = orbit32_near2(dt) near's (accel_near)
+// a step's force: accel32, within near2 = orbit32_near2(dt) near's (accel_near)
 template <class M, class Table, class Near>
 PGX_HD Acc64i orbit32_accel(const Force32 &K, const Table &table, const Near &near, const OrbitScale &s, double dt, float near2,
                             int64_t x, int64_t y, int64_t z, float &r2) {
     Acc64i a = accel32<M>(K, table, s.c, x, y, z, r2);
-    if (r2 < near2) a = near(s, dt, x, y, z);
+    if (r2 < near2) a = near(K, s, dt, x, y, z);
     return a;
 }
 
@@ -305,9 +312,9 @@ PGX_HD int64_t displacement(double v, double dt, double unit) {
     const double w = v * dt;
     return f64_to_i64(w * unit) + f64_to_i64(fma(v, dt, -w) * unit);
 }
-// whether an orbit may start at q: outside the near field, and where FP64's positions are no finer than the unit's
-PGX_HD bool orbit32_start_ok(const double *q, float near2) {
-    return fma(q[0], q[0], fma(q[1], q[1], q[2] * q[2])) >= fmax((double)near2, kOrbit32MinStart * kOrbit32MinStart);
+// whether an orbit may start at q: not where FP64's positions are much finer than the unit
+PGX_HD bool orbit32_start_ok(const double *q) {
+    return fma(q[0], q[0], fma(q[1], q[1], q[2] * q[2])) >= kOrbit32MinStart * kOrbit32MinStart;
 }
 // a displacement's drift in position units, sh = 6 + k
 PGX_HD int64_t orbit32_drift(int64_t w, int sh) {
@@ -320,17 +327,24 @@ PGX_HD int64_t orbit32_drift(int64_t w, int sh) {
 }
 
 // position q and velocity v (kpc, kpc/Myr): displacements of the first drift, v dt + a dt^2 / 2; |q| and |v dt| below the
-// scale's range, q outside the near field
-template <class M, class Table>
-PGX_HD void orbit32_start(Orbit32 &o, const Force32 &K, const Table &table, const OrbitScale &s, const double *q,
-                          const double *v, double dt, float &r2) {
+// scale's range; accel(x, y, z, r2): a position's force
+template <class Accel>
+PGX_HD void orbit32_start(Orbit32 &o, const Accel &accel, const OrbitScale &s, const double *q, const double *v, double dt,
+                          float &r2) {
     const double ux = pow2(55 - s.e), uw = pow2(61 - s.e + s.k);
-    const int64_t half = 32LL << s.k;
+    const int64_t half = 1LL << (5 + s.k);
     o.x = f64_to_i64(q[0] * ux); o.y = f64_to_i64(q[1] * ux); o.z = f64_to_i64(q[2] * ux);
-    const Acc64i a = accel32<M>(K, table, s.c, o.x, o.y, o.z, r2);
+    const Acc64i a = accel(o.x, o.y, o.z, r2);
     o.wx = displacement(v[0], dt, uw) + a.x / 2 + half;
     o.wy = displacement(v[1], dt, uw) + a.y / 2 + half;
     o.wz = displacement(v[2], dt, uw) + a.z / 2 + half;
+}
+// the same with the force on pairs of floats anywhere
+template <class M, class Table>
+PGX_HD void orbit32_start(Orbit32 &o, const Force32 &K, const Table &table, const OrbitScale &s, const double *q,
+                          const double *v, double dt, float &r2) {
+    orbit32_start(o, [&](int64_t x, int64_t y, int64_t z, float &r) { return accel32<M>(K, table, s.c, x, y, z, r); }, s, q, v,
+                  dt, r2);
 }
 
 }  // namespace pgx

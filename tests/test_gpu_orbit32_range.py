@@ -1,5 +1,5 @@
-"""The float-pair orbit's ranges on the GPU: orbits whose steps near the centre take the FP64 force, orbits that start inside
-that radius (FP64 throughout), the displacements' units (short steps, large orbits, fast ones) and the reach's end, against
+"""The float-pair orbit's ranges on the GPU: orbits whose steps near the centre take the bulge in FP64, orbits that start there
+or so near the centre that they are FP64 throughout, the units (small, large and fast orbits, short steps) and the reach's end, against
 the oracle's ph_pair_clone and with the same bits from one lane and eight lanes per clone."""
 import numpy as np
 import pytest
@@ -14,7 +14,8 @@ pytestmark = pytest.mark.gpu
 def clones(rng):
     """Circular and plunging orbits, fast and distant ones, and starts on both sides of the near field's radius."""
     out = [circular(rng, 8), circular(rng, 6, 1.2, 0.3), circular(rng, 6, 2.5, 0.3), circular(rng, 6, 0.4, 0.2),
-           circular(rng, 4, 300.0, 1.0), circular(rng, 4, 1500.0, 1.0)]
+           circular(rng, 4, 0.16, 0.02), circular(rng, 4, 300.0, 1.0), circular(rng, 4, 1500.0, 1.0),
+           circular(rng, 4, 2e5, 1.0), circular(rng, 2, 7e5, 1.0)]
     plunge = circular(rng, 10, 3.0, 0.5)
     plunge[:, 3:6] *= 0.05
     plunge[::2, 9:12] *= 0.02
