@@ -444,6 +444,7 @@ int pgx_open(int device, PgxContext **out) {
         auto init = [&]() -> int {
             CK(cudaSetDevice(device));
             CK(cudaDeviceGetAttribute(&ctx->sms, cudaDevAttrMultiProcessorCount, device));
+            ctx->mixed.sms = ctx->sms;
             if (pgx::orbit_setup(device)) return fail(ctx, PGX_E_CUDA, "pgx_open: orbit force tables");
             CK(cudaStreamCreateWithFlags(&ctx->st, cudaStreamNonBlocking));
             int lo = 0, hi = 0;

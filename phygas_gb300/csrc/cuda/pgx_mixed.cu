@@ -1000,11 +1000,11 @@ __device__ __forceinline__ double point64_at(const ScreenTables &T, int s, int c
 }
 
 // The candidates' FP64 values, bound by the FP64 pipe.  A warp takes `per` of them in turn (512; fewer when that would
-// leave the GPU's 2,432 resident warps without work), sorts them by what
+// leave resident warps, kEvalResident per SM, without work), sorts them by what
 // classify32 finds in FP32 -- nothing to do, the form at the point alone (40 % of them), everything -- into two queues in
 // shared memory and evaluates each queue 32 at a time, so that the short evaluations do not wait for long ones.
 // 4.74 M candidates of 2,000 stars x 4,087 clusters: 1.42 -> 0.92 ms.
-constexpr int kEvalWarps = 4, kEvalEntries = 512, kEvalResident = 2432, kEvalQueue = 64;
+constexpr int kEvalWarps = 4, kEvalEntries = 512, kEvalResident = 16, kEvalQueue = 64;
 __global__ void __launch_bounds__(kEvalWarps * 32) k_mx_eval64(ScreenTables T, double cut, int ne, int per,
                                                                const PossPair *__restrict__ P,
                                                                const int2 *__restrict__ E, double *__restrict__ ev,
@@ -1217,7 +1217,8 @@ int mixed_select(cudaStream_t st, const ScreenTables &T, double cut, MixedBufs &
             }
         }
         if (ne > 0) {
-            const int per = std::min(kEvalEntries, std::max(32, ne / kEvalResident / 32 * 32)), in_block = kEvalWarps * per;
+            const int per = std::min(kEvalEntries, std::max(32, ne / (kEvalResident * m.sms) / 32 * 32));
+            const int in_block = kEvalWarps * per;
             k_mx_eval64<<<(ne + in_block - 1) / in_block, kEvalWarps * 32, 0, st>>>(T, cut, ne, per, P, E, ev, es);
             launches += 1;
         }

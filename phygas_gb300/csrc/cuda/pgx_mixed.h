@@ -15,6 +15,7 @@ struct DevBuf {
 struct MixedBufs {
     DevBuf order, ub, kmin, flag, cnt, off, total, kept, cand, cand_off, ent, entq, aux, ovf;
     std::string err;
+    int sms = 1;                      // of the device
     int scan_variant = 0;             // the block filter's launch shape (scan_shape), chosen by the screen autotuner
 };
 // the block filter's launch shapes: how many, and shape v's resident blocks per SM asked of the compiler
