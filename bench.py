@@ -60,9 +60,10 @@ FLOPS_PER_PAIR_POINT = 126.0
 FLOPS_PER_BODY_STEP = 104.0
 FP64_INSTR_PER_BODY_STEP = 36.0 + 3.0 + 29.0
 # warp instructions the clone kernel issues per clone-step (two body steps on FP32 pairs and 64-bit integers, and the
-# segment's bound): smsp__inst_executed.sum of k_pair_mc_t on the 4,052-pair batch of `bench.py --mode pairs` (200 screen
-# pairs of 2,000 stars + 1 pulsar x 3,852 prefiltered clusters), 4.16e10 for 1.4905e9 clone-steps, 31.6 lanes active
-CLONE_WARP_INSTR_PER_STEP = 4.15995e10 / 1.4904824e9
+# segment's bound): smsp__inst_executed.sum of k_pair_mc_t, 4 warps a block and one clone per lane, in a separate capture of
+# the 4,052-pair batch of `bench.py --mode pairs` (200 screen pairs of 2,000 stars + 1 pulsar x 3,852 prefiltered
+# clusters), 4.10e10 for 1.4905e9 clone-steps, 31.5 lanes active
+CLONE_WARP_INSTR_PER_STEP = 4.10224e10 / 1.4904824e9
 # DRAM traffic of one k_stm_orbits launch on the whole chunk (dram__bytes_read.sum + dram__bytes_write.sum, one ncu
 # capture of `bench.py --mode screen --stars 20000 --parts 1`): 6.7 MB read + 711.9 MB of orbit output written
 ORBIT_TRAFFIC_BYTES = 718.6e6
@@ -279,7 +280,7 @@ def pair_cpu_baseline(cp, pp, n_clones=200, clusters_per_proc=24, procs=None):
                       "slowest process %.1f s" % (procs * k, k, n_clones, clone_steps, max(runs))}
 
 
-def pair_mc_measure(ctx, stars, clusters, cp, rows, want_cpu, clocks):
+def pair_mc_measure(ctx, stars, clusters, cp, rows, want_cpu, device):
     """C3-style batch: draws on the host, the autotuner on a sample of it, then the batch timed on the GPU."""
     import numpy as np
     import phygas_gb300 as pg
@@ -324,10 +325,13 @@ def pair_mc_measure(ctx, stars, clusters, cp, rows, want_cpu, clocks):
     best, table = ctx.tune_pair(*pg.draw_pair_batch(targets, ti[::25], clusters, ci[::25], ncl[::25], 0.05))
     ctx.pair(*batch)                                         # warm-up
     ms = []
-    for _ in range(2):
-        ctx.pair(*batch)
-        st = ctx.stats()
-        ms.append(st["ms_pair"])
+    with Clocks(device) as clk:                              # batches for about 2 s: several clock samples
+        t0 = time.perf_counter()
+        while len(ms) < 2 or time.perf_counter() - t0 < 2.0:
+            ctx.pair(*batch)
+            st = ctx.stats()
+            ms.append(st["ms_pair"])
+    clocks = clk.summary()
     cs = st["clone_steps"]
     # end to end: host records -> clone draws (batches of 1,024 pairs, each drawn while the GPU traces the one
     # before) -> GPU -> results, one pgx_pair_targets call
@@ -340,16 +344,19 @@ def pair_mc_measure(ctx, stars, clusters, cp, rows, want_cpu, clocks):
     rate = cs / (statistics.mean(ms) * 1e-3)
     import torch
     issue_peak = (ISSUE_PER_CLK_SM * torch.cuda.get_device_properties(0).multi_processor_count *
-                  (clocks.get("sm_mhz") or clocks.get("sm_max_mhz")) * 1e6)
+                  (clocks["sm_mhz"] or 0.0) * 1e6)
     out = {"metric": "clone-steps/s", "value": rate, "unit": "clone-steps/s", "ms_per_batch": statistics.mean(ms),
+           "batches": len(ms), "clocks": clocks,
            "workload": "%d screen pairs (p_r50 >= 0.001) + %d pulsars x %d prefiltered clusters; clones U{200,500,1000}, "
                        "dt 0.05 Myr" % (len(take), C3_PULSARS, len(pti)),
            "pairs": int(len(ti)), "clones": int(st["clones"]), "clone_steps": int(cs),
            "launch": "one captured CUDA graph (prep, persistent trace, reduce) per shape, replayed per batch",
            "roofline": {"bound": "issue", "kernel": "k_pair_mc_t", "achieved": CLONE_WARP_INSTR_PER_STEP * rate / 1e9,
                         "peak": issue_peak / 1e9, "unit": "G warp instructions/s",
-                        "frac": CLONE_WARP_INSTR_PER_STEP * rate / issue_peak,
-                        "peak_source": "4 per clock and SM at the SM clock sampled during the timed steps",
+                        "frac": CLONE_WARP_INSTR_PER_STEP * rate / issue_peak if issue_peak else None,
+                        "peak_source": "4 per clock and SM at the SM clock sampled during these batches",
+                        "achieved_source": "instructions per clone-step of a separate capture of the 2,299,100-clone batch, "
+                                           "at the rate measured here",
                         "warp_instr_per_clone_step": CLONE_WARP_INSTR_PER_STEP},
            "autotune": {"chosen": {"warps_per_block": table[best][0], "clones_per_lane": table[best][1],
                                    "min_blocks_per_sm": table[best][2]},
@@ -889,7 +896,7 @@ def main():
     pair_mc = None
     if not args.no_pair:
         try:
-            pair_mc = pair_mc_measure(ctx, stars, clusters, cp, r, rank == 0 and not args.no_cpu, clk.summary())
+            pair_mc = pair_mc_measure(ctx, stars, clusters, cp, r, rank == 0 and not args.no_cpu, local)
         except Exception as e:          # reported beside the headline, not part of it
             log("pair Monte Carlo measurement failed: %s" % e)
 
