@@ -175,8 +175,8 @@ struct Orbit {
     }
 };
 
-// mw_accel and the step on four lanes per orbit: the same operations on the same operands, so the same bits, in 32 FP64
-// warp instructions a step instead of 68.  An FP64 warp instruction costs the same with one lane active or 32, so where
+// mw_accel and the step on four lanes per orbit: the same operations on the same operands, so the same bits, in 34 FP64
+// warp instructions executed a step (ncu; 32 in the expressions) instead of 68.  An FP64 warp instruction costs the same with one lane active or 32, so where
 // there are fewer orbits than the schedulers can use lanes, an orbit's independent operations go side by side: lane 0
 // holds x and the bulge, lane 1 y and the disk, lane 2 z and the halo, lane 3 the halo's side products.  A product is
 // issued as fma(a, b, -0.0), which rounds the same.  q: the lane's coordinate (lane 3: anything finite).

@@ -13,7 +13,8 @@ struct PhResultDev {
 
 constexpr int kMcThreads = 128;
 // Batches of at most this many clones per SM take eight lanes per clone (k_pair_mc_quad): up to two warps a scheduler.
-// 2,000 steps, one lane against eight: 1 x 1,000 clones 1.86 and 1.10 ms, 4,000 2.00 and 1.60, 10,000 2.24 and 2.72.
+// 2,000 steps, one lane against eight: 1 x 1,000 clones 1.91 and 1.04 ms, 4,000 1.81 and 1.43, 6,000 1.85 and 1.47, 8,000 1.86
+// and 1.90, 10,000 1.93 and 2.46.  (The line was drawn where a slower eight-lane step crossed; it now would at 50 per SM.)
 constexpr int kMcQuadClones = 32, kMcQuadWarps = 4;
 
 // Clone Monte Carlo work: clones of pair p are [clone_off[p], clone_off[p+1]); ps = 12 doubles per clone

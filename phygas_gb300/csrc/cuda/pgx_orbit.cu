@@ -64,7 +64,7 @@ static __global__ void __launch_bounds__(128) k_stm_orbits(int N, const double *
 }
 
 // The same orbits on four lanes each (quad_accel: the same bits), 8 orbits per warp, one warp per block.  For objects few
-// enough that every warp has a scheduler to itself: a step is then 32 dependent FP64 warp instructions where one lane
+// enough that every warp has a scheduler to itself: a step is then 34 FP64 warp instructions in a row where one lane
 // per orbit takes 68, at 64 cycles each with the SM's other schedulers idle.
 static __global__ void __launch_bounds__(32) k_stm_orbits_quad(int N, const double *__restrict__ ps0,
                                                                const int *__restrict__ npts, int nmax,
@@ -93,7 +93,7 @@ static __global__ void __launch_bounds__(32) k_stm_orbits_quad(int N, const doub
 }
 
 // Four lanes per orbit while 7 N orbits at 8 a warp leave each scheduler at most one warp (694 objects on 152 SMs): 1 star
-// 4.7 -> 2.96 ms, 301 stars 4.8 -> 3.01 ms.  Beyond, a scheduler would issue 2 x 32 instructions a step for 16 orbits where
+// 4.7 -> 2.96 ms, 301 stars 4.8 -> 3.01 ms.  Beyond, a scheduler would issue 2 x 34 instructions a step for 16 orbits where
 // one lane per orbit issues 68 for 32.  There, blocks of one warp while the warps are fewer than the schedulers, so that
 // they spread over the SMs (four schedulers share a pipe that serves each at 76 cycles an instruction, three at 64):
 // 2,000 stars 5.3 -> 4.8 ms.  max_blocks > 0: a grid of that many blocks of 128 at most, to run beside other work.
@@ -284,7 +284,7 @@ __device__ __noinline__ Approach trace_clone64(const double *__restrict__ ps, in
 }
 
 // Four clones by a warp in FP64, eight lanes each (the same bits): lanes 0-3 of the eight trace the target, 4-7 the cluster
-// (quad_accel).  ps, steps and dt are the eight's clone's; every lane of the warp calls.  A step takes 32 FP64 instructions
+// (quad_accel).  ps, steps and dt are the eight's clone's; every lane of the warp calls.  A step takes 34 FP64 instructions
 // where trace_clone64 takes 136, so up to three such passes end sooner.
 __device__ __noinline__ Approach trace_clone64_eights(const double *__restrict__ ps, int steps, double dt) {
     const unsigned all = 0xffffffffu, eight = 0xffu << (threadIdx.x & 24u);
@@ -738,7 +738,7 @@ cudaError_t launch_coarse_tracks(cudaStream_t st, int N, const double *ps, const
 }
 
 // The clones of a warp that take the FP64 trace: n steps of each lane's clone (0: none; every lane calls).  Up to twelve are
-// traced four at a time (3 x 32 FP64 instructions a step at most), more lane by lane (136).  One after the other, as it was,
+// traced four at a time (3 x 34 FP64 instructions a step at most), more lane by lane (136).  One after the other, as it was,
 // 10 pairs x 400 clones at steps of 0.2 Myr took 8.5 ms, four at a time 2.3.
 __device__ __forceinline__ void trace_fp64(const double *ps, int n, int steps, double dt, Approach &r) {
     const unsigned all = 0xffffffffu;
