@@ -228,7 +228,8 @@ __device__ double safe_u(double value, double e) {
 // Where the clones of pair q begin in its stream: at[slot[q] + k] = the state before its k-th successful clone,
 // m[q] = how many succeed of n_clones[q] (as ph_pair_draw takes them: a target or a cluster that fails all its tries
 // drops the clone).  Lane l of a warp looks at the clone l after the next one as if none before it drew again; the
-// clones before the first that does are settled together, that one is walked through, and the rest look again.
+// clones before the first that does are settled together, that one's tries are taken side by side, and the rest look again
+// (2,000 clones whose tries all fail: 21 ms, 354 with the tries one after the other on every lane).
 __global__ void k_pair_streams(int n_pairs, const PhTarget *__restrict__ t, const int *__restrict__ ti,
                                const PhCluster *__restrict__ c, const int *__restrict__ ci,
                                const int *__restrict__ n_clones, const uint64_t *__restrict__ seed,
@@ -250,6 +251,14 @@ __global__ void k_pair_streams(int n_pairs, const PhTarget *__restrict__ t, cons
     int k = 0;                                                    // clones that succeeded
     auto uniform = [](uint64_t g) { return Rng{g}.uniform(); };   // the first deviate of the Gaussian at g
     auto gauss = [](uint64_t g) { return Rng{g}.gauss(); };
+    // how many of the tries from s on fail before one succeeds (kTries: all of them), a lane each
+    auto failed = [&](auto succeeds) {
+        for (int i = 0; i < kTries; i += 32) {
+            const unsigned yes = __ballot_sync(all, i + lane < kTries && succeeds(after_gaussians(s, i + lane)));
+            if (yes) return i + __ffs(yes) - 1;
+        }
+        return kTries;
+    };
     for (int j = 0; j < n;) {
         const uint64_t g = after_gaussians(s, 8 * lane);
         bool bad = false;
@@ -264,13 +273,14 @@ __global__ void k_pair_streams(int n_pairs, const PhTarget *__restrict__ t, cons
         k += good;
         j += good;
         s = after_gaussians(s, 8 * good);
-        if (again && j < n) {                                     // clone j, try by try (every lane alike)
+        if (again && j < n) {                                     // clone j: its tries side by side
             const uint64_t start = s;
-            int a = 0, b = 0;
-            while (a < kTries && !(target_plx(tq, gauss(s)) > 0)) { a++; s = after_gaussians(s, 1); }
+            const int a = failed([&](uint64_t g) { return target_plx(tq, gauss(g)) > 0; });
+            s = after_gaussians(s, a);
             if (a < kTries) {
                 s = after_gaussians(s, 4);
-                while (b < kTries && !(cluster_dist(cq, gauss(s)) > 0)) { b++; s = after_gaussians(s, 1); }
+                const int b = failed([&](uint64_t g) { return cluster_dist(cq, gauss(g)) > 0; });
+                s = after_gaussians(s, b);
                 if (b < kTries) {
                     s = after_gaussians(s, 4);
                     if (lane == 0) o[k] = start;
