@@ -240,7 +240,7 @@ __global__ void k_pair_streams(int n_pairs, const PhTarget *__restrict__ t, cons
     if (q >= n_pairs) return;                                     // the whole warp: uniform
     const PhTarget &tq = t[ti[q]];
     const PhCluster &cq = c[ci[q]];
-    if (lane < 2) frames[q].f[lane] = lane ? frame_of(cq.ra, cq.dec) : frame_of(tq.ra, tq.dec);
+    if (lane < 2) frames[q].f[lane] = frame_of(lane ? cq.ra : tq.ra, lane ? cq.dec : tq.dec);
     // a target without a parallax has a positive distance times an exponential within FP64's range
     const double ut = tq.plx > 0 ? safe_u(tq.plx, tq.e_plx)
                                  : (tq.dist_pc > 1e-100 && tq.dist_pc < 1e100 && fabs(tq.e_lndist) < 10.0 ? 0.0 : 2.0);
