@@ -185,7 +185,8 @@ int pgx_tracks(PgxContext *ctx, int n, const double *ps, const int *npts, double
  * force is evaluated on pairs of floats (2^-47 relative), within 12 |dt| kpc of the centre (dt in Myr; at least 0.4) its
  * dominant part, the bulge's, in FP64, for 0.01 <= |dt| <= 0.125 Myr, starts 0.15 kpc and more from the centre and orbits within 10^6 kpc; everything
  * else is traced in FP64.  Over that range the orbits end no further from exact arithmetic than FP64 steps do (5 to 50
- * times nearer on galactic orbits); the two differ by FP64's rounding, some 1e-13 of the results. */
+ * times nearer on galactic orbits); the two differ by FP64's rounding, some 1e-13 of the results.  With PHYGAS_PAIR_FP64=1
+ * in the environment when a context is opened, its pgx_pair and pgx_pair_targets trace every clone in FP64 steps. */
 int pgx_pair(PgxContext *ctx, int n_pairs, const int *clone_off, const double *ps, const int *steps,
              const double *dt, const double *r50_pc, const double *rtot_pc, PhResult *res, double *clone_out);
 

@@ -116,6 +116,7 @@ struct PgxContext {
     long n_rows = 0;
     // pair Monte Carlo
     Buf p_off, p_ps, p_steps, p_dt, p_r50, p_rt, p_items, p_q, p_cres, p_res, p_params;
+    bool pair_fp64 = false;                    // PHYGAS_PAIR_FP64=1: every clone in FP64 steps
     int mc_variant = 0;                        // launch shape of the clone kernel (pgx_tune_pair picks it)
     int mc_blocks_per_sm = 0;                  // > 0: the persistent clone kernels on at most this many blocks per SM
     const int *mc_busy = nullptr;              // set: the cap applies only while *mc_busy is nonzero at a launch
@@ -438,6 +439,7 @@ int pgx_open(int device, PgxContext **out) {
     ctx->device = device;
     if (const char *e = getenv("PHYGAS_SCAN_BLOCKS")) ctx->scan_blocks = atoi(e) != 0;
     if (const char *e = getenv("PHYGAS_SCAN_TMA")) ctx->scan_tma = atoi(e) != 0;
+    if (const char *e = getenv("PHYGAS_PAIR_FP64")) ctx->pair_fp64 = atoi(e) != 0;
     if (const char *e = getenv("PHYGAS_FAIL_ALLOC_AT")) ctx->fail_alloc_at = atol(e);
     int rc = 0;
     {
@@ -1506,6 +1508,7 @@ int pair_run(PgxContext *ctx, int variant, int n_pairs, const int *clone_off, co
     Pp.dt = P<double>(ctx->p_dt); Pp.r50_pc = P<double>(ctx->p_r50); Pp.rtot_pc = P<double>(ctx->p_rt);
     Pp.items = P<int4>(ctx->p_items); Pp.qhead = P<int>(ctx->p_q);
     Pp.cres = P<double>(ctx->p_cres); Pp.res = P<pgx::PhResultDev>(ctx->p_res);
+    Pp.fp64 = ctx->pair_fp64;
     ctx->stats = PgxStats();
     // prep, trace and the reduction of pairs of at most 1024 clones; the parameters travel by copy: the graph's kernels
     // read them from p_params

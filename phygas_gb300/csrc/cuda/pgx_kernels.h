@@ -27,6 +27,7 @@ struct McPairs {
     const double *r50_pc, *rtot_pc;
     const int4 *items;        // (pair, first clone, count, -)
     int *qhead;               // queue head (set by k_mc_prep)
+    int fp64;                 // nonzero: every clone in FP64 steps
     double *cres;             // [3][n_clones]: best (kpc), tbest (Myr), vbest (kpc/Myr)
     PhResultDev *res;         // per pair
 };

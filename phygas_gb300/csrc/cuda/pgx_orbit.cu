@@ -517,15 +517,15 @@ struct Clone32 {
     Near32 n;
     float rmax, near2;       // r2 limits
     bool ok;
-    // false: not an orbit for these units (traced in FP64)
-    __device__ __forceinline__ bool start(const double *__restrict__ ps, int steps, double dt) {
+    // false: not an orbit for these units, or FP64 asked for (traced in FP64)
+    __device__ __forceinline__ bool start(const double *__restrict__ ps, int steps, double dt, bool fp64) {
         double p[12];
 #pragma unroll
         for (int j = 0; j < 12; j++) p[j] = ps[j];
         n.pend = false;
         n.tie = 0;
         near2 = orbit32_near2(dt);
-        ok = clone_scale(p, steps, dt, s);
+        ok = !fp64 && clone_scale(p, steps, dt, s);
         if (!ok) {                                            // (stepped along where its lane has another clone)
             a = b = Orbit32{};
             K = Force32{};
@@ -614,12 +614,12 @@ struct QuadClone32 {
         const Orbit32 a = gather(x0, w, 0), b = gather(x0, w, 4);
         return vertex64(a, b, force32_constants<MwModel32>(dt, s), s, i, dt);
     }
-    __device__ __forceinline__ void start(const double *__restrict__ ps, int steps, double dt, int role) {
+    __device__ __forceinline__ void start(const double *__restrict__ ps, int steps, double dt, int role, bool fp64) {
         double p[12];
 #pragma unroll
         for (int j = 0; j < 12; j++) p[j] = ps[j];
         near2 = orbit32_near2(dt);
-        ok = clone_scale(p, steps, dt, s);
+        ok = !fp64 && clone_scale(p, steps, dt, s);
         if (!ok) {                                            // (traced along with its warp, and again in FP64)
             s = OrbitScale{0x1p-23f, 0};
             near2 = 0.f;
@@ -772,7 +772,7 @@ __device__ __forceinline__ Approach trace_clone(bool active, const double *__res
     Clone32 c;
     c.ok = c.n.pend = false;
     c.n.tie = 0;
-    if (active && c.start(ps, steps, dt)) {
+    if (active && c.start(ps, steps, dt, false)) {
 #pragma unroll 1
         for (int i = 1; i <= steps; i++) c.step(i, dt);
     }
@@ -924,7 +924,7 @@ __global__ void __launch_bounds__(WARPS * 32, MINB > 1 ? MINB : 16 / (WARPS * CP
 #pragma unroll
         for (int j = 0; j < CPL; j++) {
             const int e = lane + 32 * j < it.z ? lane + 32 * j : min(lane, it.z - 1);
-            any |= c[j].start(P.ps + (size_t)(it.y + e) * 12, steps, dt);
+            any |= c[j].start(P.ps + (size_t)(it.y + e) * 12, steps, dt, P.fp64 != 0);
         }
         if (any) {
 #pragma unroll 1
@@ -958,7 +958,7 @@ __global__ void __launch_bounds__(kMcQuadWarps * 32) k_pair_mc_quad(const McPair
         const int p = it.x, steps = P.steps[p], cc = it.y + min(e, it.z - 1);
         const double dt = P.dt[p];
         QuadClone32 c;
-        c.start(P.ps + (size_t)cc * 12, steps, dt, role);
+        c.start(P.ps + (size_t)cc * 12, steps, dt, role, P.fp64 != 0);
         if (__any_sync(0xffffffffu, c.ok)) {
 #pragma unroll 1
             for (int i = 1; i <= steps; i++) c.step(i, dt, role);
